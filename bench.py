@@ -1158,7 +1158,10 @@ def work_model(diag, fused):
     (a divide or square root counts as one flop, an FMA as two):
       leaf Jacobi     (12 s + 15) flops per rotation, s(s-1)/2 rotations a
                       sweep, summed over the leaves with the sweeps each
-                      leaf's half-warp ran
+                      leaf's half-warp ran; leaves solved one eigenpair per
+                      lane: per pair ten evaluations of det(T - x) of 8
+                      (s - 1) flops, 26 s for the vector and its residual,
+                      4 s^2 for the orthogonality correction
       secular         8 flops per pole-root pair and sweep; sweeps per root
                       = its iterations + the initial midpoint sweep
       Loewner         4 flops per pair (inner merges only)
@@ -1168,8 +1171,10 @@ def work_model(diag, fused):
     nlev = len(levels)
     leaves = diag["leaf_count"]
     s = 16
-    sweeps = diag.get("leaf_sweeps_sum") or leaves * diag["leaf_sweeps_max"]
+    sweeps = diag["leaf_sweeps_sum"]
     leaf = sweeps * (s * (s - 1) / 2) * (12 * s + 15)
+    if sweeps == 0:  # no leaf took Jacobi
+        leaf = leaves * s * (10 * 8 * (s - 1) + 26 * s + 4 * s * s)
     per = []
     for k, lv in enumerate(levels):
         kk = max(lv["dd_after_sum"], 1)

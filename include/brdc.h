@@ -180,7 +180,8 @@ typedef struct brdc_diagnostics {
     int n;
     int levels;
     int leaf_count;
-    int leaf_sweeps_max;     /* Jacobi sweeps of the slowest leaf */
+    int leaf_sweeps_max;     /* Jacobi sweeps of the slowest leaf that took them
+                                (0: every leaf was solved pair by pair) */
     int leaf_sweeps_sum;     /* Jacobi sweeps summed over the leaves */
     brdc_level_diagnostics level[BRDC_MAX_LEVELS];
 } brdc_diagnostics;

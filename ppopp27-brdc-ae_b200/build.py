@@ -55,7 +55,7 @@ def build(force: bool = False, verbose: bool = False) -> str:
             cmd.insert(1, "-Xptxas=-v")
         subprocess.run(cmd, check=True)
     cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
-    hdeps = [os.path.join(CSRC, "host_check.cpp"), os.path.join(CSRC, "brdc_secular.cuh")]
+    hdeps = [os.path.join(CSRC, f) for f in ("host_check.cpp", "brdc_secular.cuh", "brdc_leaf.cuh")]
     if force or _stale(HOSTLIB, hdeps):
         subprocess.run(
             [cxx, "-O2", "-fPIC", "-shared", "-std=c++17", "-o", HOSTLIB,

@@ -703,10 +703,17 @@ brdc_status run_forest(brdc_handle h, const HostForest &hf, const Layout &L,
     const long long leaf_per = 2LL * kLeafWarps; // leaves per block
     long long leaf_grid = (hf.leaves + leaf_per - 1) / leaf_per;
     leaf_grid = std::max<long long>(1, std::min<long long>(leaf_grid, (long long)h->sm_count * 16));
+    bool leaves_done = true;
     if (L.ckpt) {
         k_leaf_full<<<(unsigned)leaf_grid, kLeafWarps * 32, 0, s>>>(a, hf.leaves);
         BRDC_CUDA(h, "brdc.leaf_full", cudaGetLastError());
         ++h->launches;
+    } else if (sub == 0) {
+        k_leaf<<<(unsigned)leaf_grid, kLeafWarps * 32, 0, s>>>(a, hf.leaves);
+        BRDC_CUDA(h, "brdc.leaf", cudaGetLastError());
+        ++h->launches;
+    } else {
+        leaves_done = false; // by the subtrees
     }
     if (sub > 0) {
         SubArgs A{};
@@ -722,7 +729,7 @@ brdc_status run_forest(brdc_handle h, const HostForest &hf, const Layout &L,
         A.out_l = (fused & 1) ? w.nl : w.cl;
         A.levels = sub;
         A.ckpt = L.ckpt ? 1 : 0;
-        A.leaves_done = L.ckpt ? 1 : 0;
+        A.leaves_done = leaves_done ? 1 : 0;
         long long subs = 0;
         for (int b = 0; b < hf.B; ++b) {
             subs += subtrees_of(hf.lev[b], sub);
@@ -748,11 +755,6 @@ brdc_status run_forest(brdc_handle h, const HostForest &hf, const Layout &L,
             std::swap(a.w.cl, a.w.nl);
         }
     } else {
-        if (!L.ckpt) {
-            k_leaf<<<(unsigned)leaf_grid, kLeafWarps * 32, 0, s>>>(a, hf.leaves);
-            BRDC_CUDA(h, "brdc.leaf", cudaGetLastError());
-            ++h->launches;
-        }
         mark(h, 2);
         h->fused_levels = 0;
     }

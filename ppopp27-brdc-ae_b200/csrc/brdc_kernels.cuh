@@ -28,6 +28,7 @@
 #include <cstdint>
 
 #include "brdc_common.cuh"
+#include "brdc_leaf.cuh"
 #include "brdc_secular.cuh"
 
 namespace brdc {
@@ -48,11 +49,20 @@ struct KArgs {
 };
 
 // ------------------------------------------------------------------ leaves
-// Leaves of <= 16 rows, two per warp (one per half-warp), by parallel
-// cyclic Jacobi, as the reference solves its leaves by Jacobi
-// (gpu/src/tridiag_solver_leaf.cuh:56-123, one thread per leaf there).
+// Leaves of <= 16 rows, two per warp (one per half-warp): one eigenpair per
+// lane (leaf_pairs, brdc_leaf.cuh), and where that leaves a leaf (nearly
+// diagonal ones, eigenvalues too close) parallel cyclic Jacobi, as the
+// reference solves its leaves (gpu/src/tridiag_solver_leaf.cuh:56-123, one
+// thread per leaf there).
 //
-// Lane x of a half-warp owns column x of the 16x16 leaf matrix in
+// Why not Jacobi throughout: it exchanges whole columns of a full 16 x 16
+// matrix for six sweeps of 15 rounds, 79 shuffles each, which bounded it
+// (100 us for the 4096 leaves of n = 65,536, one wave).  The eigenpairs need
+// about 1500 FP64 instructions a lane and a few shuffles.  Measured on B200:
+// a solve of n = 100 130 -> 85 us, normal 4,096 310 -> 259, uniform 65,536
+// 702 -> 625; the leaves of the 1024-matrix fit step 4.5 -> 0.4 ms.
+//
+// Jacobi: Lane x of a half-warp owns column x of the 16x16 leaf matrix in
 // registers, stored XOR-skewed: reg[j] = A[x^j][x].  Sweep m = 1..15 of the
 // XOR tournament pairs index x with x^m (every pair exactly once per sweep),
 // so in round m: the diagonal is reg[0], the entry to annihilate is reg[m],
@@ -65,6 +75,9 @@ struct KArgs {
 // applied on load.  Output: ascending eigenvalues with the first and last
 // rows in that order.
 constexpr int kLeafWarps = 4;
+// resident blocks per SM (at 4 a thread has 128 registers): 2, 3 and 4 took
+// 573.5, 572.2 and 567.9 us of a normal 65,536 solve with its leaves in k_leaf
+constexpr int kLeafBlocks = 4;
 constexpr unsigned kFull = 0xffffffffu;
 
 // The arithmetic of a leaf rotation, spelled out (explicit FMAs and rounded
@@ -72,6 +85,25 @@ constexpr unsigned kFull = 0xffffffffu;
 // and leaf_round_v produce bit for bit the same matrix and rows.
 __device__ __forceinline__ double leaf_rot(double c, double x, double sgs, double y) {
     return fma(c, x, __dmul_rn(sgs, y)); // c x + (sg s) y
+}
+
+// The plane rotation (c, sn) that annihilates apq, t = sn / c.  A leaf of
+// one warp waits for each of its roundings, so the quotients are
+// reciprocals (brdc_rcp, whose operands are normal here) and 1/sqrt is one
+// function: against three divisions and two square roots a round, the
+// slowest leaves of clustered 49,151 went from 67 to 55 us.
+__device__ __forceinline__ void leaf_angle(double app, double aqq, double apq, double *c,
+                                           double *sn, double *t) {
+    const double den = 2.0 * apq;
+    const double theta = fabs(den) > 0x1p-900 ? (aqq - app) * brdc_rcp(den) : (aqq - app) / den;
+    if (fabs(theta) > 1.0e150) {
+        *t = 0.5 / theta;
+    } else {
+        const double r = brdc_rcp(fabs(theta) + sqrt(fma(theta, theta, 1.0)));
+        *t = theta >= 0.0 ? r : -r;
+    }
+    *c = rsqrt(fma(*t, *t, 1.0));
+    *sn = __dmul_rn(*t, *c);
 }
 
 template <int M>
@@ -89,17 +121,9 @@ __device__ __forceinline__ void leaf_round(double (&a)[16], double &v0,
     const double app = isp ? mydiag : odiag;
     const double aqq = isp ? odiag : mydiag;
     double c = 1.0, sn = 0.0, t = 0.0;
-    int rot = 0;
-    if (fabs(apq) > th) {
-        const double theta = (aqq - app) / (2.0 * apq);
-        if (fabs(theta) > 1.0e150) {
-            t = 0.5 / theta;
-        } else {
-            t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(fma(theta, theta, 1.0)));
-        }
-        c = 1.0 / sqrt(fma(t, t, 1.0));
-        sn = __dmul_rn(t, c);
-        rot = 1;
+    const bool rot = fabs(apq) > th;
+    if (rot) {
+        leaf_angle(app, aqq, apq, &c, &sn, &t);
     }
     // columns: B = A J  (col p: c*col_p - s*col_q, col q: s*col_p + c*col_q)
     const double sgx = isp ? -1.0 : 1.0;
@@ -135,22 +159,34 @@ __device__ __forceinline__ void leaf_round(double (&a)[16], double &v0,
     }
 }
 
-__device__ __forceinline__ double half_max(double v) {
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) {
-        v = fmax(v, __shfl_xor_sync(kFull, v, o));
+// Rounds M..15 of a sweep.  A round in which no lane's entry exceeds th turns
+// nothing and is passed over.  The leaves that come here are mostly nearly
+// diagonal ones, with many such rounds (clustered 4,096: 238 -> 221 us a solve;
+// uniform leaves, when they still came here, lost 5% of the subtree to the
+// votes).
+template <int M>
+__device__ __forceinline__ void leaf_sweep(double (&a)[16], double &v0, double &v1, int x,
+                                           double th) {
+    if (__any_sync(kFull, fabs(a[M]) > th)) {
+        leaf_round<M>(a, v0, v1, x, th);
     }
-    return v;
+    if constexpr (M < 15) {
+        leaf_sweep<M + 1>(a, v0, v1, x, th);
+    }
 }
 
-// Jacobi solve of one leaf by a half-warp (lane x of the half owns column x;
-// both halves of the warp call this together, the other half on its own
-// leaf or with s = 0).  Returns the leaf's eigenvalue of rank x (ascending;
-// +inf for x >= s) with the first and last entries of its eigenvector, and
-// the number of sweeps taken.
-__device__ inline int leaf_solve(const KArgs &a, const LeafGeom &G, int s, int x,
-                                 double *key_out, double *v0_out, double *v1_out) {
-    const double eps = DBL_EPSILON;
+// What lane x of a half-warp returns of its leaf: the eigenvalue of rank x
+// (ascending; +inf or unset for x >= s), the first and last entries of its
+// eigenvector, and the Jacobi sweeps taken.
+struct LeafRow {
+    double key, v0, v1;
+    int sweeps;
+};
+
+// Row x of leaf G: its diagonal with the cuts' corrections, and the moduli
+// of its couplings to the rows below and above.
+__device__ __forceinline__ void leaf_load(const KArgs &a, const LeafGeom &G, int s, int x,
+                                          double *d, double *e_below, double *e_above) {
     double dx = 0.0, ex = 0.0, exm1 = 0.0;
     if (x < s) {
         const double sc = inst_scale(a.w, G.inst);
@@ -168,6 +204,16 @@ __device__ inline int leaf_solve(const KArgs &a, const LeafGeom &G, int s, int x
             exm1 = sc * fabs(a.E[G.gstart + x - 1]);
         }
     }
+    *d = dx;
+    *e_below = ex;
+    *e_above = exm1;
+}
+
+// Jacobi solve of one leaf by a half-warp (lane x of the half owns column x
+// and passes leaf_load's values; both halves of the warp call this together,
+// the other half on its own leaf or with s = 0).
+__device__ __forceinline__ LeafRow leaf_solve(double dx, double ex, double exm1, int s, int x) {
+    const double eps = DBL_EPSILON;
     double reg[16];
     const int jup = x ^ (x + 1);
     const int jdn = x ^ (x - 1);
@@ -194,21 +240,7 @@ __device__ inline int leaf_solve(const KArgs &a, const LeafGeom &G, int s, int x
         if (!__any_sync(kFull, off > th)) {
             break;
         }
-        leaf_round<1>(reg, v0, v1, x, th);
-        leaf_round<2>(reg, v0, v1, x, th);
-        leaf_round<3>(reg, v0, v1, x, th);
-        leaf_round<4>(reg, v0, v1, x, th);
-        leaf_round<5>(reg, v0, v1, x, th);
-        leaf_round<6>(reg, v0, v1, x, th);
-        leaf_round<7>(reg, v0, v1, x, th);
-        leaf_round<8>(reg, v0, v1, x, th);
-        leaf_round<9>(reg, v0, v1, x, th);
-        leaf_round<10>(reg, v0, v1, x, th);
-        leaf_round<11>(reg, v0, v1, x, th);
-        leaf_round<12>(reg, v0, v1, x, th);
-        leaf_round<13>(reg, v0, v1, x, th);
-        leaf_round<14>(reg, v0, v1, x, th);
-        leaf_round<15>(reg, v0, v1, x, th);
+        leaf_sweep<1>(reg, v0, v1, x, th);
     }
 
     // bitonic sort of (eigenvalue, column) within the half-warp
@@ -235,10 +267,38 @@ __device__ inline int leaf_solve(const KArgs &a, const LeafGeom &G, int s, int x
             }
         }
     }
-    *key_out = key;
-    *v0_out = v0;
-    *v1_out = v1;
-    return sweep;
+    return LeafRow{key, v0, v1, sweep};
+}
+
+// One leaf by a half-warp: leaf_pairs, or Jacobi where that leaves the leaf.
+// put(key, v0, v1) stores lane x's eigenvalue of rank x with the first and
+// last entries of its eigenvector.  Returns the Jacobi sweeps taken (0 for
+// none).  The first result is stored before Jacobi starts, so that nothing
+// of it weighs on Jacobi's registers.
+template <class Put>
+__device__ __forceinline__ int leaf_rows(const KArgs &a, const LeafGeom &G, LeafScratch &B, int s,
+                                         int x, Put put) {
+    bool done;
+    {
+        double dx, ex, exm1;
+        leaf_load(a, G, s, x, &dx, &ex, &exm1);
+        double key, v0, v1, vf[kLeafN];
+        done = leaf_pairs<false>(B, dx, ex, s, x, &key, &v0, &v1, vf);
+        if (done && x < s) {
+            put(key, v0, v1);
+        }
+    }
+    if (!__any_sync(kFull, !done && s > 0)) {
+        return 0;
+    }
+    const int sj = done ? 0 : s;
+    double dx, ex, exm1;
+    leaf_load(a, G, sj, x, &dx, &ex, &exm1);
+    const LeafRow r = leaf_solve(dx, ex, exm1, sj, x);
+    if (x < sj) {
+        put(r.key, r.v0, r.v1);
+    }
+    return sj > 0 ? r.sweeps : 0;
 }
 
 // leaf_round on the whole eigenvector matrix (lane x holds column x in v):
@@ -258,17 +318,9 @@ __device__ __forceinline__ void leaf_round_v(double (&a)[16], double (&v)[16],
     const double app = isp ? mydiag : odiag;
     const double aqq = isp ? odiag : mydiag;
     double c = 1.0, sn = 0.0, t = 0.0;
-    int rot = 0;
-    if (fabs(apq) > th) {
-        const double theta = (aqq - app) / (2.0 * apq);
-        if (fabs(theta) > 1.0e150) {
-            t = 0.5 / theta;
-        } else {
-            t = (theta >= 0.0 ? 1.0 : -1.0) / (fabs(theta) + sqrt(fma(theta, theta, 1.0)));
-        }
-        c = 1.0 / sqrt(fma(t, t, 1.0));
-        sn = __dmul_rn(t, c);
-        rot = 1;
+    const bool rot = fabs(apq) > th;
+    if (rot) {
+        leaf_angle(app, aqq, apq, &c, &sn, &t);
     }
     const double sgx = isp ? -1.0 : 1.0;
     double b[16];
@@ -301,6 +353,17 @@ __device__ __forceinline__ void leaf_round_v(double (&a)[16], double (&v)[16],
     }
 }
 
+// leaf_sweep with leaf_round_v.
+template <int M>
+__device__ __forceinline__ void leaf_sweep_v(double (&a)[16], double (&v)[16], int x, double th) {
+    if (__any_sync(kFull, fabs(a[M]) > th)) {
+        leaf_round_v<M>(a, v, x, th);
+    }
+    if constexpr (M < 15) {
+        leaf_sweep_v<M + 1>(a, v, x, th);
+    }
+}
+
 // leaf_solve with the whole eigenvector matrix, for a checkpointing
 // forward (the adjoint of a leaf needs all of it): the same sweeps and
 // rotations, so rows 0 and s-1 of v are bit for bit leaf_solve's v0 and v1,
@@ -309,23 +372,8 @@ __device__ __forceinline__ void leaf_round_v(double (&a)[16], double (&v)[16],
 __device__ inline int leaf_solve_full(const KArgs &a, const LeafGeom &G, int s, int x,
                                       double *key_out, double (&v)[16]) {
     const double eps = DBL_EPSILON;
-    double dx = 0.0, ex = 0.0, exm1 = 0.0;
-    if (x < s) {
-        const double sc = inst_scale(a.w, G.inst);
-        dx = sc * a.D[G.gstart + x];
-        if (x == 0 && G.gstart > G.istart) {
-            dx -= sc * fabs(a.E[G.gstart - 1]);
-        }
-        if (x == s - 1 && G.gstart + s < G.iend) {
-            dx -= sc * fabs(a.E[G.gstart + s - 1]);
-        }
-        if (x + 1 < s) {
-            ex = sc * fabs(a.E[G.gstart + x]);
-        }
-        if (x >= 1) {
-            exm1 = sc * fabs(a.E[G.gstart + x - 1]);
-        }
-    }
+    double dx, ex, exm1;
+    leaf_load(a, G, s, x, &dx, &ex, &exm1);
     double reg[16];
     const int jup = x ^ (x + 1);
     const int jdn = x ^ (x - 1);
@@ -347,21 +395,7 @@ __device__ inline int leaf_solve_full(const KArgs &a, const LeafGeom &G, int s, 
         if (!__any_sync(kFull, off > th)) {
             break;
         }
-        leaf_round_v<1>(reg, v, x, th);
-        leaf_round_v<2>(reg, v, x, th);
-        leaf_round_v<3>(reg, v, x, th);
-        leaf_round_v<4>(reg, v, x, th);
-        leaf_round_v<5>(reg, v, x, th);
-        leaf_round_v<6>(reg, v, x, th);
-        leaf_round_v<7>(reg, v, x, th);
-        leaf_round_v<8>(reg, v, x, th);
-        leaf_round_v<9>(reg, v, x, th);
-        leaf_round_v<10>(reg, v, x, th);
-        leaf_round_v<11>(reg, v, x, th);
-        leaf_round_v<12>(reg, v, x, th);
-        leaf_round_v<13>(reg, v, x, th);
-        leaf_round_v<14>(reg, v, x, th);
-        leaf_round_v<15>(reg, v, x, th);
+        leaf_sweep_v<1>(reg, v, x, th);
     }
     // bitonic sort of (eigenvalue, column) within the half-warp, as leaf_solve
     double key = (x < s) ? reg[0] : INFINITY;
@@ -399,7 +433,7 @@ __device__ inline int leaf_solve_full(const KArgs &a, const LeafGeom &G, int s, 
 // The leaves of a checkpointing forward: leaf_solve_full, then the leaf
 // outputs as k_leaf writes them plus, for the adjoint, every eigenvalue
 // (leafl) and eigenvector (leafv, 16 entries per column) in sorted order.
-__global__ void __launch_bounds__(kLeafWarps * 32)
+__global__ void __launch_bounds__(kLeafWarps * 32, kLeafBlocks)
     k_leaf_full(KArgs a, long long total_leaves) {
     pdl_begin();
     if (halted(a.w.hdr)) {
@@ -408,6 +442,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32)
     const int lane = threadIdx.x & 31;
     const int x = lane & 15;
     const int half = lane >> 4;
+    __shared__ __align__(16) LeafScratch sB[kLeafWarps * 2];
     int sweeps_max = 0, sweeps_sum = 0;
     const long long pairs = (total_leaves + 1) / 2;
     for (long long pr = (long long)blockIdx.x * kLeafWarps + (threadIdx.x >> 5); pr < pairs;
@@ -421,10 +456,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32)
             s = G.s;
         }
         double key, v[16];
-        const int sweep = leaf_solve_full(a, G, s, x, &key, v);
-        sweeps_max = sweeps_max > sweep ? sweeps_max : sweep;
-        sweeps_sum += (x == 0 && s > 0) ? sweep : 0;
-        if (x < s) {
+        auto put = [&]() {
             const long long o = G.gstart + x;
             double vlast = 0.0;
 #pragma unroll
@@ -440,6 +472,22 @@ __global__ void __launch_bounds__(kLeafWarps * 32)
                 a.w.cf[o] = v[0];
                 a.w.cl[o] = vlast;
             }
+        };
+        double dx, ex, exm1, u0, u1;
+        leaf_load(a, G, s, x, &dx, &ex, &exm1);
+        const bool done = leaf_pairs<true>(sB[(threadIdx.x >> 5) * 2 + half], dx, ex, s, x, &key,
+                                           &u0, &u1, v);
+        if (done && x < s) {
+            put();
+        }
+        if (__any_sync(kFull, !done && s > 0)) {
+            const int sj = done ? 0 : s;
+            const int sweep = leaf_solve_full(a, G, sj, x, &key, v);
+            sweeps_max = sweeps_max > sweep ? sweeps_max : sweep;
+            sweeps_sum += (x == 0 && sj > 0) ? sweep : 0;
+            if (x < sj) {
+                put();
+            }
         }
     }
     sweeps_sum = __reduce_add_sync(kFull, sweeps_sum);
@@ -449,7 +497,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32)
     }
 }
 
-__global__ void __launch_bounds__(kLeafWarps * 32)
+__global__ void __launch_bounds__(kLeafWarps * 32, kLeafBlocks)
     k_leaf(KArgs a, long long total_leaves) {
     pdl_begin();
     if (halted(a.w.hdr)) {
@@ -458,6 +506,7 @@ __global__ void __launch_bounds__(kLeafWarps * 32)
     const int lane = threadIdx.x & 31;
     const int x = lane & 15;
     const int half = lane >> 4;
+    __shared__ __align__(16) LeafScratch sB[kLeafWarps * 2];
     int sweeps_max = 0, sweeps_sum = 0;
     const long long pairs = (total_leaves + 1) / 2;
     for (long long pr = (long long)blockIdx.x * kLeafWarps + (threadIdx.x >> 5); pr < pairs;
@@ -470,20 +519,19 @@ __global__ void __launch_bounds__(kLeafWarps * 32)
             G = leaf_geom(a.F, leaf);
             s = G.s;
         }
-        double key, v0, v1;
-        const int sweep = leaf_solve(a, G, s, x, &key, &v0, &v1);
-        sweeps_max = sweeps_max > sweep ? sweeps_max : sweep;
-        sweeps_sum += (x == 0 && s > 0) ? sweep : 0;
-        if (x < s) {
-            const long long o = G.gstart + x;
-            if (G.top) {
-                a.W[o] = key * inst_unscale(a.w, G.inst);
-            } else {
-                a.w.cd[o] = key;
-                a.w.cf[o] = v0;
-                a.w.cl[o] = v1;
-            }
-        }
+        const int sweep = leaf_rows(
+            a, G, sB[(threadIdx.x >> 5) * 2 + half], s, x, [&](double key, double v0, double v1) {
+                const long long o = G.gstart + x;
+                if (G.top) {
+                    a.W[o] = key * inst_unscale(a.w, G.inst);
+                } else {
+                    a.w.cd[o] = key;
+                    a.w.cf[o] = v0;
+                    a.w.cl[o] = v1;
+                }
+            });
+        sweeps_max = max(sweeps_max, sweep);
+        sweeps_sum += x == 0 ? sweep : 0;
     }
     sweeps_sum = __reduce_add_sync(kFull, sweeps_sum);
     if (lane == 0 && sweeps_max > 0) {

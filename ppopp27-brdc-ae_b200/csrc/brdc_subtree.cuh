@@ -74,6 +74,14 @@ struct SubSmem {
     int it_sum, it_max, it_failed;
 };
 
+// The leaves' scratch lies over md .. rlam (cd, cf and cl take their results).
+static_assert(2 * sizeof(LeafScratch) * SubSmem<256>::kSubWarps <=
+                      offsetof(SubSmem<256>, rf) - offsetof(SubSmem<256>, md) &&
+                  2 * sizeof(LeafScratch) * SubSmem<512>::kSubWarps <=
+                      offsetof(SubSmem<512>, rf) - offsetof(SubSmem<512>, md) &&
+                  offsetof(SubSmem<256>, md) % 16 == 0 && offsetof(SubSmem<512>, md) % 16 == 0,
+              "leaf scratch");
+
 // Exclusive scan of one int per thread over the CTA; ex[kSubRows] = total.
 template <int kSubRows>
 __device__ inline void sub_scan(SubSmem<kSubRows> &S, int v) {
@@ -208,11 +216,9 @@ __global__ void __launch_bounds__(kSubRows, 512 / kSubRows) k_subtree(SubArgs A)
                 LG.inst = b;
                 s = LG.s;
             }
-            double key, v0, v1;
-            const int sw = leaf_solve(a, LG, s, xl, &key, &v0, &v1);
-            sweeps_max = sweeps_max > sw ? sweeps_max : sw;
-            sweeps_sum += (xl == 0 && s > 0) ? sw : 0;
-            if (xl < s) {
+            // scratch: the level arrays from md on, idle until the leaves are done
+            LeafScratch *B = reinterpret_cast<LeafScratch *>(S.md) + 2 * warp + half;
+            const int sw = leaf_rows(a, LG, *B, s, xl, [&](double key, double v0, double v1) {
                 const int o = (int)(LG.gstart - gsub) + xl;
                 if (LG.top) {
                     a.W[LG.gstart + xl] = key * wsc;
@@ -221,7 +227,9 @@ __global__ void __launch_bounds__(kSubRows, 512 / kSubRows) k_subtree(SubArgs A)
                     S.cf[o] = v0;
                     S.cl[o] = v1;
                 }
-            }
+            });
+            sweeps_max = max(sweeps_max, sw);
+            sweeps_sum += xl == 0 ? sw : 0;
         }
         sweeps_sum = __reduce_add_sync(kFull, sweeps_sum);
         if (lane == 0 && sweeps_max > 0) {
