@@ -1451,6 +1451,47 @@ __device__ inline void secular_span(SecSums &sum, const SecRoot &st, int j0,
     }
 }
 
+// Sums of one root over the poles l, l + tpr, ... of K in shared memory; the
+// brackets of the warp's roots lie in [pmin, r1].  Up to kOneLoop poles a
+// lane one loop serves both sides of the bracket: the segment loops' starts
+// and remainders, and lanes whose segments differ in length, cost more than
+// its two extra FP64 instructions a pole.  Measured on B200 (cycles of a
+// sweep, segments -> one loop, 512 threads): 32 poles a lane 4935 -> 2990,
+// 63 6121 -> 5093, 106 8291 -> 7956 and in its first sweep 14771 -> 15694;
+// Toeplitz merges at 128 and more poles a lane lost 15% by it.
+constexpr int kOneLoop = 64;
+
+__device__ inline SecTot secular_shared(const SecRoot &st, const double *pd, const double *pz,
+                                        int K, int l, int tpr, int pmin, int r1) {
+    if (K <= kOneLoop * tpr) {
+        SecTot sum{};
+#pragma unroll 4
+        for (int j = l; j < K; j += tpr) {
+            sec_accum_any(sum, st, j, pd[j], pz[j]);
+        }
+        return sum;
+    }
+    SecSums sum;
+    sec_zero(sum);
+    secular_span(sum, st, 0, K, l, tpr, pmin, r1, [&](int u, double *du, double *zu) {
+        *du = pd[u];
+        *zu = pz[u];
+    });
+    return sec_total(sum);
+}
+
+__device__ inline void sums_reduce(SecTot &sum, int tpr) {
+    for (int o = tpr >> 1; o > 0; o >>= 1) {
+        SecTot other;
+        other.sum = __shfl_xor_sync(0xffffffffu, sum.sum, o);
+        other.mag = __shfl_xor_sync(0xffffffffu, sum.mag, o);
+        other.dpsi = __shfl_xor_sync(0xffffffffu, sum.dpsi, o);
+        other.dphi = __shfl_xor_sync(0xffffffffu, sum.dphi, o);
+        other.err = __shfl_xor_sync(0xffffffffu, sum.err, o);
+        sec_combine(sum, other);
+    }
+}
+
 __device__ inline void sums_reduce(SecSums &sum, int tpr) {
     for (int o = tpr >> 1; o > 0; o >>= 1) {
         SecSums other;

@@ -377,17 +377,11 @@ __device__ void level_roots(LvlSmem &S, cooperative_groups::cluster_group &cl, c
             } else {
                 st.stage = 2;
             }
-            const int pmin = r < K - 2 ? r : K - 2;
             for (;;) {
-                SecSums sum;
-                sec_zero(sum);
+                SecTot sum{};
                 const bool live = act && st.stage != 2;
                 if (live) {
-                    secular_span(sum, st, 0, K, l2, tp, pmin, r + 1,
-                                 [&](int u, double *du, double *zu) {
-                                     *du = S.pd[u];
-                                     *zu = S.pz[u];
-                                 });
+                    sum = secular_shared(st, S.pd, S.pz, K, l2, tp, r < K - 2 ? r : K - 2, r + 1);
                 }
                 sums_reduce(sum, tp);
                 if (live) {

@@ -108,6 +108,19 @@ __host__ __device__ inline void sec_zero(SecSums &s) {
     s.err = 0.0;
 }
 
+// A root's sums as sec_after_sweep reads them.
+struct SecTot {
+    double sum;  // psi + phi
+    double mag;  // phi - psi: the sum of the terms' moduli
+    double dpsi; // sum_{j < p} z_j^2 / delta_j^2
+    double dphi; // sum_{j > p+1} z_j^2 / delta_j^2
+    double err;  // running-sum rounding bound
+};
+
+__host__ __device__ inline SecTot sec_total(const SecSums &s) {
+    return SecTot{s.psi + s.phi, s.phi - s.psi, s.dpsi, s.dphi, s.err};
+}
+
 struct SecRoot {
     // problem (fixed)
     int i;         // root index
@@ -261,6 +274,37 @@ __host__ __device__ inline void sec_accum_right(SecSums &s, const SecRoot &r,
     s.err += s.phi;
 }
 
+// One term of a sweep whose lanes' roots have their brackets anywhere in
+// it, added to both sides' totals at once: a term's sign is its delta's, so
+// the signed sum and the sum of moduli hold psi and phi between them, and
+// only the squares need to know the side.  Poles p and p+1 add nothing
+// (their t is made a denormal by its high word).  Two FP64 instructions
+// more than the one-sided form, but one loop: where a warp's roots spread
+// over a merge, a left and a right loop each run as long as their longest
+// lane.
+__host__ __device__ inline double sec_high(double x, bool clear, int high) {
+#ifdef __CUDA_ARCH__
+    return __hiloint2double(clear ? high : __double2hiint(x), __double2loint(x));
+#else
+    return clear ? (high != 0 ? 1.0 : 0.0) : x;
+#endif
+}
+
+__host__ __device__ inline void sec_accum_any(SecTot &s, const SecRoot &r, int j, double dj,
+                                              double zj) {
+    const bool skip = (unsigned)(j - r.p) < 2u;
+    const bool left = j < r.p;
+    const double z = fabs(zj);
+    const double delta = sec_high((dj - r.eorg_d) - r.etau, skip, 0x3ff00000);
+    const double t = sec_high(z * brdc_rcp(delta), skip, 0);
+    s.sum = fma(z, t, s.sum);
+    s.mag = fma(z, fabs(t), s.mag);
+    const double tl = sec_high(t, !left, 0), tr = sec_high(t, left, 0);
+    s.dpsi = fma(tl, tl, s.dpsi);
+    s.dphi = fma(tr, tr, s.dphi);
+    s.err += s.mag;
+}
+
 // Combine partial sums of two lanes (the tree adds its own rounding).  Every
 // operation is commutative in (a, b), so the lanes of a butterfly reduction
 // end with bit-identical sums and take identical branches afterwards.
@@ -270,6 +314,14 @@ __host__ __device__ inline void sec_combine(SecSums &a, const SecSums &b) {
     a.phi = a.phi + b.phi;
     a.dphi = a.dphi + b.dphi;
     a.err = (a.err + b.err) + (fabs(a.psi) + a.phi);
+}
+
+__host__ __device__ inline void sec_combine(SecTot &a, const SecTot &b) {
+    a.sum = a.sum + b.sum;
+    a.mag = a.mag + b.mag;
+    a.dpsi = a.dpsi + b.dpsi;
+    a.dphi = a.dphi + b.dphi;
+    a.err = (a.err + b.err) + a.mag;
 }
 
 __host__ __device__ inline double sec_clamp_tau(double t, double lo, double hi) {
@@ -283,7 +335,7 @@ __host__ __device__ inline double sec_clamp_tau(double t, double lo, double hi) 
 // new stage (2 once converged or failed).  A root still unconverged after
 // max_iter iterations, or whose secular function evaluates to NaN, is
 // finished with r.failed set.
-__host__ __device__ inline int sec_after_sweep(SecRoot &r, const SecSums &s,
+__host__ __device__ inline int sec_after_sweep(SecRoot &r, const SecTot &s,
                                                double eps, int max_iter = kSecularMaxIter) {
     if (r.stage == 2) {
         return 2;
@@ -291,33 +343,25 @@ __host__ __device__ inline int sec_after_sweep(SecRoot &r, const SecSums &s,
     if (r.stage == 0) {
         // Initial guess from the two bracketing poles with the rest of the
         // sum frozen at the evaluation point.
-        const double c = r.rhoinv + s.psi + s.phi;
+        const double c = r.rhoinv + s.sum;
         if (!r.last) {
+            // root in (d_p, mid) with origin p, or in [mid, d_q) with origin
+            // p+1: the second is the first mirrored (sg = -1)
             const double del = r.dq - r.dp;
             const double mid = r.etau;
-            const double w = c + r.zp2 / (-mid) + r.zq2 / ((r.dq - r.dp) - mid);
-            double tau;
-            if (w > 0.0) {
-                // root in (d_p, mid): origin p
-                r.org = r.p;
-                r.dorg = r.dp;
-                r.lo = 0.0;
-                r.hi = mid;
-                const double a = c * del + r.zp2 + r.zq2;
-                const double b = r.zp2 * del;
-                const double disc = sqrt(fabs(a * a - 4.0 * b * c));
-                tau = (a > 0.0) ? 2.0 * b / (a + disc) : (a - disc) / (2.0 * c);
-            } else {
-                // root in [mid, d_q): origin p+1
-                r.org = r.p + 1;
-                r.dorg = r.dq;
-                r.lo = -mid;
-                r.hi = 0.0;
-                const double a = c * del - r.zp2 - r.zq2;
-                const double b = r.zq2 * del;
-                const double disc = sqrt(fabs(a * a + 4.0 * b * c));
-                tau = (a < 0.0) ? 2.0 * b / (a - disc) : -(a + disc) / (2.0 * c);
-            }
+            const double rm = brdc_rcp(mid);
+            const double w = c - r.zp2 * rm + r.zq2 * brdc_rcp(del - mid);
+            const bool left = w > 0.0;
+            const double sg = left ? 1.0 : -1.0;
+            r.org = left ? r.p : r.p + 1;
+            r.dorg = left ? r.dp : r.dq;
+            r.lo = left ? 0.0 : -mid;
+            r.hi = left ? mid : 0.0;
+            const double a = sg * (c * del) + (r.zp2 + r.zq2);
+            const double b = (left ? r.zp2 : r.zq2) * del;
+            const double disc = sqrt(fabs(a * a - sg * (4.0 * b * c)));
+            double tau = (a > 0.0 ? sg * (2.0 * b) : a - disc) *
+                         brdc_rcp(a > 0.0 ? a + disc : 2.0 * c);
             tau = sec_clamp_tau(tau, r.lo, r.hi);
             // Two safeguarded Newton steps on the model that also keeps the
             // slope of the rest of the sum at the midpoint,
@@ -424,31 +468,21 @@ __host__ __device__ inline int sec_after_sweep(SecRoot &r, const SecSums &s,
     const double tq = r.zq2 * rq;
     const double dtp = tp * rp;    // z_p^2 / delta_p^2
     const double dtq = tq * rq;
-    const double psi_f = s.psi + tp;
-    const double phi_f = s.phi + tq;
     const double dpsi_f = s.dpsi + dtp;
     const double dphi_f = s.dphi + dtq;
-    const double w = r.rhoinv + psi_f + phi_f;
+    const double w = (r.rhoinv + s.sum) + tp + tq;
     const double dw = dpsi_f + dphi_f;
 
     double erretm;
     if (!r.last) {
-        double psil = s.psi, phil = s.phi, err = s.err, torg;
-        if (r.org == r.p) {
-            phil += tq;
-            err += phil;
-            torg = tp;
-        } else {
-            psil += tp;
-            err += fabs(psil);
-            torg = tq;
-        }
-        erretm = 8.0 * (phil - psil) + err + 2.0 * r.rhoinv +
-                 3.0 * fabs(torg) + fabs(tau) * dw;
+        // the far side's bracket term joins the running sums last
+        const bool left = r.org == r.p;
+        const double side = left ? 0.5 * (s.mag + s.sum) + tq : 0.5 * (s.mag - s.sum) - tp;
+        erretm = 8.0 * (s.mag + (left ? tq : -tp)) + (s.err + fabs(side)) + 2.0 * r.rhoinv +
+                 3.0 * fabs(left ? tp : tq) + fabs(tau) * dw;
     } else {
-        const double psil = s.psi + tp;
-        const double err = s.err + fabs(psil);
-        erretm = 8.0 * (-tq - psil) + err - tq + r.rhoinv + fabs(tau) * dw;
+        const double side = 0.5 * (s.mag - s.sum) - tp;
+        erretm = 8.0 * (s.mag - tp - tq) + (s.err + fabs(side)) - tq + r.rhoinv + fabs(tau) * dw;
     }
 
     if (!(w == w)) {
@@ -489,54 +523,47 @@ __host__ __device__ inline int sec_after_sweep(SecRoot &r, const SecSums &s,
     }
     r.prevw = w;
 
+    // The step of either model, and of the last root's, is a root of the
+    // same quadratic c eta^2 - a eta + b = 0 with its own c; the roots of a
+    // warp take different ones, so each choice is a select and the square
+    // root and the reciprocal are taken once.  (The same numbers as branches
+    // with a root and a quotient each; a warp went through most of those.)
+    const bool mw = r.last || (r.swtch && r.iter > 1); // middle way
+    const bool orgati = r.org == r.p;
+    // fixed weight: (d_p - d_q) (z_p / delta_p)^2 or its mirror image
+    const double m1 = !mw && orgati ? dlq : dlp;
+    const double n1 = mw ? dpsi_f : dw;
+    const double m2 = mw ? dlq : orgati ? r.dp - r.dq : r.dq - r.dp;
+    const double n2 = mw ? dphi_f : orgati ? dtp : dtq;
+    double c = w - m1 * n1 - m2 * n2;
+    c = r.last && r.iter == 1 ? fabs(c) : c;
+    const double a = (dlp + dlq) * w - dlp * dlq * dw;
+    const double b = dlp * dlq * w;
     double eta;
-    if (!r.last) {
-        double c;
-        if (r.swtch && r.iter > 1) {
-            c = w - dlp * dpsi_f - dlq * dphi_f;
-        } else if (r.org == r.p) {
-            // fixed weight: (d_p - d_q) * (z_p / delta_p)^2
-            c = w - dlq * dw - (r.dp - r.dq) * dtp;
+    if (c == 0.0) {
+        if (r.last) {
+            eta = r.hi - tau;
         } else {
-            c = w - dlp * dw - (r.dq - r.dp) * dtq;
-        }
-        const double a = (dlp + dlq) * w - dlp * dlq * dw;
-        const double b = dlp * dlq * w;
-        if (c == 0.0) {
             double aa = a;
             if (aa == 0.0) {
-                if (r.swtch && r.iter > 1) {
+                if (mw) {
                     aa = dlp * dlp * dpsi_f + dlq * dlq * dphi_f;
-                } else if (r.org == r.p) {
+                } else if (orgati) {
                     aa = r.zp2 + dlq * dlq * dw;
                 } else {
                     aa = r.zq2 + dlp * dlp * dw;
                 }
             }
             eta = b * brdc_rcp(aa);
-        } else if (a <= 0.0) {
-            eta = (a - sqrt(fabs(a * a - 4.0 * b * c))) * brdc_rcp(2.0 * c);
-        } else {
-            eta = 2.0 * b * brdc_rcp(a + sqrt(fabs(a * a - 4.0 * b * c)));
-        }
-        if (w * eta >= 0.0) {
-            eta = -w * brdc_rcp(dw);
         }
     } else {
-        const double c0 = w - dlp * dpsi_f - dlq * dphi_f;
-        const double c = (r.iter == 1) ? fabs(c0) : c0;
-        const double a = (dlp + dlq) * w - dlp * dlq * dw;
-        const double b = dlp * dlq * w;
-        if (c == 0.0) {
-            eta = r.hi - tau;
-        } else if (a >= 0.0) {
-            eta = (a + sqrt(fabs(a * a - 4.0 * b * c))) * brdc_rcp(2.0 * c);
-        } else {
-            eta = 2.0 * b * brdc_rcp(a - sqrt(fabs(a * a - 4.0 * b * c)));
-        }
-        if (w * eta > 0.0) {
-            eta = -w * brdc_rcp(dw);
-        }
+        const double root = sqrt(fabs(a * a - 4.0 * b * c));
+        const double sr = r.last ? root : -root;
+        const bool direct = r.last ? a >= 0.0 : a <= 0.0;
+        eta = (direct ? a + sr : 2.0 * b) * brdc_rcp(direct ? 2.0 * c : a - sr);
+    }
+    if (r.last ? w * eta > 0.0 : w * eta >= 0.0) {
+        eta = -w * brdc_rcp(dw);
     }
     double tnew = tau + eta;
     if (!(tnew > r.lo && tnew < r.hi)) {
@@ -547,6 +574,11 @@ __host__ __device__ inline int sec_after_sweep(SecRoot &r, const SecSums &s,
     r.etau = tnew;
     r.eorg_d = r.dorg;
     return 1;
+}
+
+__host__ __device__ inline int sec_after_sweep(SecRoot &r, const SecSums &s, double eps,
+                                               int max_iter = kSecularMaxIter) {
+    return sec_after_sweep(r, sec_total(s), eps, max_iter);
 }
 
 // Host/serial driver: solve root i of (d, z, rho) with K >= 1 poles by

@@ -503,17 +503,11 @@ __global__ void __launch_bounds__(kSubRows, 512 / kSubRows) k_subtree(SubArgs A)
                 } else {
                     st.stage = 2;
                 }
-                const int pmin = rr < Kr - 2 ? rr : Kr - 2;
                 for (;;) {
-                    SecSums sum;
-                    sec_zero(sum);
+                    SecTot sum{};
                     const bool live = act && st.stage != 2;
                     if (live) {
-                        secular_span(sum, st, 0, Kr, l2, lanes, pmin, rr + 1,
-                                     [&](int u, double *du, double *zu) {
-                                         *du = pd[u];
-                                         *zu = pz[u];
-                                     });
+                        sum = secular_shared(st, pd, pz, Kr, l2, lanes, rr < Kr - 2 ? rr : Kr - 2, rr + 1);
                     }
                     sums_reduce(sum, lanes);
                     if (live) {
@@ -547,15 +541,9 @@ __global__ void __launch_bounds__(kSubRows, 512 / kSubRows) k_subtree(SubArgs A)
             } else {
                 st.stage = 2;
             }
-            SecSums sum;
-            sec_zero(sum);
+            SecTot sum{};
             if (act) {
-                const int pmin = rr < Kr - 2 ? rr : Kr - 2;
-                secular_span(sum, st, 0, Kr, l2, tp, pmin, rr + 1,
-                             [&](int u, double *du, double *zu) {
-                                 *du = pd[u];
-                                 *zu = pz[u];
-                             });
+                sum = secular_shared(st, pd, pz, Kr, l2, tp, rr < Kr - 2 ? rr : Kr - 2, rr + 1);
             }
             sums_reduce(sum, tp);
             if (act) {

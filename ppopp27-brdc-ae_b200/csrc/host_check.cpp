@@ -21,6 +21,33 @@ extern "C" int brdc_host_secular_root_capped(int K, const double *d, const doubl
                                   DBL_EPSILON, max_iter);
 }
 
+// The same root by sweeps of sec_accum_any (both sides in one loop), dealt to
+// `lanes` lanes and combined as the kernels' butterfly does.
+extern "C" int brdc_host_secular_root_any(int K, const double *d, const double *z, double rho,
+                                          double znorm2, int i, int lanes, int *org, double *tau,
+                                          int *failed) {
+    brdc::SecRoot r;
+    brdc::sec_init(r, i, K, d, z, rho, znorm2);
+    int sweeps = 0;
+    while (r.stage != 2) {
+        brdc::SecTot t[32] = {};
+        for (int j = 0; j < K; ++j) {
+            brdc::sec_accum_any(t[j % lanes], r, j, d[j], z[j]);
+        }
+        for (int o = lanes >> 1; o > 0; o >>= 1) {
+            for (int l = 0; l < o; ++l) {
+                brdc::sec_combine(t[l], t[l + o]);
+            }
+        }
+        ++sweeps;
+        brdc::sec_after_sweep(r, t[0], DBL_EPSILON);
+    }
+    *org = r.org;
+    *tau = r.tau;
+    *failed = r.failed;
+    return sweeps;
+}
+
 // One leaf of s rows (d, e >= 0, scaled to a norm in [0.5, 1)) as
 // leaf_pairs solves it, its lanes in turn: eigenvalues, vectors (s x s,
 // vector i in row i), the largest residual, |F| and evaluations of a lane.
