@@ -20,6 +20,7 @@
 
 #include "../../include/brdc_lapack.h"
 #include "brdc_backward.cuh"
+#include "brdc_box.cuh"
 #include "brdc_level.cuh"
 #include "brdc_vectors.cuh"
 #include "brdc_subtree.cuh"
@@ -605,10 +606,53 @@ int launch_sweeps(brdc_handle h, const HostForest &hf, const KArgs &a, cudaStrea
     return 1;
 }
 
-// One fused level (k_level), then k_sweeps for its merges with more than
-// kLvlMaxK poles (it returns at once when there are none; it is not launched
-// where no merge has more rows than that).  Returns the number of kernels
-// launched.
+// Resident k_box blocks per SM, once per device; 0 when the device has no
+// cooperative launch.
+int box_per_sm(int device) {
+    static int cached[64];
+    static bool done[64];
+    if (device < 0 || device >= 64) {
+        return 0;
+    }
+    if (!done[device]) {
+        int coop = 0, nb = 0;
+        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+        if (coop == 0 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+                             &nb, k_box, kSweepThreads, 0) != cudaSuccess) {
+            cudaGetLastError();
+            nb = 0;
+        }
+        cached[device] = nb;
+        done[device] = true;
+    }
+    return cached[device];
+}
+
+// The merges of level a.k that k_level leaves: one cooperative k_box.
+// Returns as launch_sweeps.
+int launch_boxes(brdc_handle h, const HostForest &hf, const KArgs &a, cudaStream_t s) {
+    const int nb = box_per_sm(h->device);
+    if (nb <= 0) {
+        return -1;
+    }
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(nb * h->sm_count));
+    cfg.blockDim = dim3(kSweepThreads);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, k_box, a, h->has_lowner[a.k], (long long)hf.total_n);
+    mark(h, 4 + 4 * a.k);
+    mark(h, 5 + 4 * a.k);
+    mark(h, 6 + 4 * a.k);
+    return 1;
+}
+
+// One fused level (k_level), then k_box for the merges it leaves (it returns
+// at once when there are none).  Returns the number of kernels launched.
 int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, bool ckpt,
                        cudaStream_t s) {
     const int k = a0.k;
@@ -626,9 +670,12 @@ int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, boo
     }
     const int C = 1 << q;
     KArgs a = a0;
-    a.big_k = kLvlMaxK;
-    // a plan is needed only where a merge can keep more than kLvlMaxK poles
-    const bool big = mmax > kLvlMaxK;
+    // k_box takes merges with more than kBoxMinK poles on the levels that
+    // launch it: those of a batch, where one more launch is nothing, and those
+    // that may hold merges k_level cannot take.  (Launched for nothing it
+    // costs a level 4 us.)
+    const bool big = mmax > (hf.B > 1 ? kBoxMinK : kLvlMaxK);
+    a.big_k = big ? kBoxMinK : kLvlMaxK;
     a.plan_inline = big && a.nodes <= kLvlThreads ? 1 : 0;
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = cluster_config((unsigned)(a.nodes * C), C, s, at);
@@ -646,13 +693,13 @@ int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, boo
     }
     mark(h, 3 + 4 * k);
     if (big) {
-        const int ns = launch_sweeps(h, hf, a, s);
+        const int ns = launch_boxes(h, hf, a, s);
         if (ns < 0) {
             return -1;
         }
         n += ns;
     } else {
-        // no merge of this level can keep more than kLvlMaxK poles
+        // k_level takes every merge of this level
         mark(h, 4 + 4 * k);
         mark(h, 5 + 4 * k);
         mark(h, 6 + 4 * k);

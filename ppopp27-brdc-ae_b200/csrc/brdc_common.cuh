@@ -88,11 +88,11 @@ struct LevelCtl {
     int items_w;     // warp work items of the level
     int items_c;     // CTA work items of the level
     int total_k;
-    int nbig;        // merges k_level left to the sweep kernels (K > kLvlMaxK)
+    int nbig;        // merges k_level left to k_box (K > kLvlMaxK)
     unsigned bar_count; // grid barrier of k_sweeps: arrivals, generation
     unsigned bar_gen;
     int citem;       // next CTA-role item of the secular phase (taken by atomicAdd)
-    int pad_ctl;
+    int box;         // poles per box of the merges k_box takes
     double work_w;   // pole-root pairs (sum K^2) of the warp-role merges
     double work_c;   // and of the CTA-role merges
 };

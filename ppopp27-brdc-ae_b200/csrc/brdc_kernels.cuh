@@ -25,6 +25,7 @@
 #include <cooperative_groups.h>
 
 #include <cfloat>
+#include <climits>
 #include <cstdint>
 
 #include "brdc_common.cuh"
@@ -601,6 +602,24 @@ __global__ void __launch_bounds__(256) k_merge(KArgs a, long long total_n) {
     }
 }
 
+constexpr int kWarpsPerBlock = kSweepThreads / 32;
+
+// Poles per box of k_box's merges of up to kmax poles (brdc_box.cuh): p K / b
+// terms once against about 4 sweeps of 3 b terms; up to 8192 poles also
+// enough boxes for the GPU.  Measured on B200 (Toeplitz): 65,536 5.75 ms at
+// 64 and 128, 5.26 at 128 and 256, 16,384 1.30 ms at 64, 1.31 at 128.
+__host__ __device__ inline int box_poles(int kmax) {
+    return kmax <= 8192 ? 64 : kmax <= 16384 ? 128 : 256;
+}
+// Merges of more poles than this are k_box's where it runs: it takes half
+// the terms, and every SM shares them (Toeplitz 16,384 1.37 ms at 1024, 1.30
+// at 512 and at 256; a batch of 512 up to 2048 rows 2.10, 1.66, 1.63 ms).
+constexpr int kBoxMinK = 512;
+// Lanes per root there at most: a lane should have two dozen of the 3 b near
+// poles (Toeplitz 16,384, two merges of 8192 poles: 860 us at 16 lanes, 798
+// at 8, 750 at 4; one of 4096 poles is faster at 8).
+constexpr int kBoxMaxLanes = 8;
+
 // Work plan of the sweep kernels for level a.k, from the node scalars the
 // deflation wrote: the level diagnostics, lanes per root, and the item
 // tables.  Merges with K <= kWarpMaxK are served one warp per work item;
@@ -610,13 +629,17 @@ __global__ void __launch_bounds__(256) k_merge(KArgs a, long long total_n) {
 template <int T>
 __device__ void level_plan(const KArgs &a, double *red, int *iscan) {
     const Ws &w = a.w;
+    // after k_level (big_k > 0) k_box takes every item: runs of roots in the
+    // warp role's tables, boxes of poles in the CTA role's
+    const bool boxes = a.big_k > 0;
+    const int wmax = boxes ? INT_MAX : kWarpMaxK;
     double tkw = 0.0, tkc = 0.0, cw = 0.0, cc = 0.0, qw = 0.0, qc = 0.0;
     double skz = 0.0, sk = 0.0, sk2 = 0.0, kmax = 0.0;
     for (int i = threadIdx.x; i < a.nodes; i += T) {
         const int kk = __ldcg(w.nK + i);
         const int kz = __ldcg(w.nKz + i);
         // nodes with K <= big_k get no items (finished by k_level, or empty)
-        if (kk > a.big_k && kk > kWarpMaxK) {
+        if (kk > a.big_k && kk > wmax) {
             tkc += kk;
             cc += 1.0;
             qc += (double)kk * (double)kk;
@@ -670,6 +693,14 @@ __device__ void level_plan(const KArgs &a, double *red, int *iscan) {
         cap <<= 1;
     }
     tpr_c = tpr_c < cap ? tpr_c : cap;
+    if (boxes) {
+        // k_box: one wave of its grid (a quarter of the default target)
+        tpr_w = 1;
+        while (tpr_w < kBoxMaxLanes && 2.0 * tpr_w * tkw <= 0.25 * a.lanes_target) {
+            tpr_w <<= 1;
+        }
+    }
+    const int box = box_poles((int)kmax);
     const int Rw = 32 / tpr_w;
     const int Rc = kSweepThreads / tpr_c;
     // each thread owns a contiguous run of nodes: serial prefix of its run,
@@ -680,10 +711,11 @@ __device__ void level_plan(const KArgs &a, double *red, int *iscan) {
     int sw = 0, sc = 0;
     for (int i = i0; i < i1; ++i) {
         const int kk = __ldcg(w.nK + i);
-        if (kk > a.big_k && kk > kWarpMaxK) {
+        if (kk > a.big_k && kk > wmax) {
             sc += (kk + Rc - 1) / Rc;
         } else if (kk > a.big_k) {
             sw += (kk + Rw - 1) / Rw;
+            sc += boxes ? kk / box : 0;
         }
     }
     int carry_w, carry_c;
@@ -693,10 +725,11 @@ __device__ void level_plan(const KArgs &a, double *red, int *iscan) {
         const int kk = __ldcg(w.nK + i);
         w.pref_w[i] = rw;
         w.pref_c[i] = rc;
-        if (kk > a.big_k && kk > kWarpMaxK) {
+        if (kk > a.big_k && kk > wmax) {
             rc += (kk + Rc - 1) / Rc;
         } else if (kk > a.big_k) {
             rw += (kk + Rw - 1) / Rw;
+            rc += boxes ? kk / box : 0;
         }
     }
     __syncthreads();
@@ -720,10 +753,11 @@ __device__ void level_plan(const KArgs &a, double *red, int *iscan) {
         c->tpr_c = tpr_c;
         c->items_w = carry_w;
         c->items_c = carry_c;
+        c->box = box;
         c->total_k = (int)(tkw + tkc);
         c->work_w = qw;
         c->work_c = qc;
-        w.hdr->diag[a.k].threads_per_root = carry_c > 0 ? tpr_c : tpr_w;
+        w.hdr->diag[a.k].threads_per_root = carry_c > 0 && !boxes ? tpr_c : tpr_w;
     }
 }
 
@@ -1542,7 +1576,6 @@ __device__ inline int block_role_setup(uint64_t *bars) {
 // ---------------------------------------------------------------- roots
 // Blocks [0, cta_blocks) serve the CTA-role merges, the others the warp-role
 // merges (8 warps per block, each on its own work item).
-constexpr int kWarpsPerBlock = kSweepThreads / 32;
 
 // The phases below are device functions over the grid's two roles, run back
 // to back by k_sweeps.  CTA-role blocks set up their two mbarriers once (ph
@@ -2120,8 +2153,7 @@ __device__ inline bool grid_barrier(WsHeader *h, LevelCtl *c) {
 
 // Roots, Loewner weights, boundary rows and placement of one level in one
 // cooperative launch: the four phases above separated by grid barriers
-// instead of kernel boundaries.  After k_level (big_k > 0) it returns at
-// once when the level plan has no items: k_level finished every merge.
+// instead of kernel boundaries, for levels that run per-level kernels.
 // The roles split the grid in proportion to their pole-root pairs in the
 // plan (all blocks to the role that has items when only one has; `tiles` =
 // 0: the launch has no tile memory and every block takes the warp role).  `rows` = 0 skips the
@@ -2137,9 +2169,6 @@ __global__ void __launch_bounds__(kSweepThreads)
     WsHeader *h = a.w.hdr;
     LevelCtl *ctl = &h->lvl[a.k];
     const int iw = __ldcg(&ctl->items_w), ic = __ldcg(&ctl->items_c);
-    if (a.big_k > 0 && iw + ic == 0) {
-        return;
-    }
     int cta_blocks = 0;
     if (tiles && ic > 0) {
         cta_blocks = (int)gridDim.x;

@@ -16,10 +16,10 @@
 // order, rotations, the secular state machine, tie order of the placement),
 // so deflation and placement decide exactly as they do; only the lanes that
 // share a root's sweep differ, which moves the sums' rounding.  A node with
-// more than kLvlMaxK poles stops after its deflation and is counted in the
-// level's nbig; the last CTA then builds the level plan for exactly those
-// nodes (big_k = kLvlMaxK), and k_sweeps finishes them (it returns at once
-// when there are none).  Every write lands where the per-level kernels put
+// more than big_k poles (at most kLvlMaxK) stops after its deflation and is
+// counted in the level's nbig; the last CTA then builds the level plan for
+// exactly those nodes, and k_box finishes them (it returns at once when
+// there are none).  Every write lands where the per-level kernels put
 // it, so the workspace slices of a checkpointed solve serve the adjoint
 // unchanged.
 #pragma once
@@ -515,7 +515,7 @@ __device__ void level_roots(LvlSmem &S, cooperative_groups::cluster_group &cl, c
     }
 }
 
-// The level plan for the merges k_level leaves to k_sweeps: taken by the
+// The level plan for the merges k_level leaves to k_box: taken by the
 // last CTA of the launch (every node's scalars are written before its CTAs
 // take their tickets), and only when there are such merges.
 template <int T>
@@ -690,15 +690,15 @@ __global__ void __launch_bounds__(T, 1) k_level(KArgs a) {
         atomicMax(&dg->dd_after_max, K);
         atomicAdd((unsigned long long *)&dg->dd_after_sq_sum,
                   (unsigned long long)K * (unsigned long long)K);
-        if (K > kLvlMaxK) {
+        if (K > a.big_k) {
             atomicAdd(&w.hdr->lvl[a.k].nbig, 1);
         }
     }
-    if (K > kLvlMaxK) {
+    if (K > a.big_k) {
         // no CTA leaves while a peer may still read its shared memory
         cl.sync();
         level_ticket<T>(a, S);
-        return; // k_sweeps finishes this node
+        return; // k_box finishes this node
     }
 
     // ------------------------------------------------ roots
