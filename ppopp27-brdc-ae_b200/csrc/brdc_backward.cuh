@@ -42,7 +42,6 @@ struct BArgs {
     int k;
     int nodes;
     long long level_rows; // rows of the instances merging at this level
-    int lanes_target;     // threads the per-row sweeps aim to keep busy
 };
 
 __device__ inline double sgn(double x) { return (double)((x > 0.0) - (x < 0.0)); }
@@ -370,84 +369,98 @@ __global__ void __launch_bounds__(kSweepThreads) k_bw_poles(BArgs a) {
 //      dL/domega = z_p sum_j (1/N_j)/delta_pj^2
 //                  (gf_m f'_j + gl_m l'_j - gf_j f_m - gl_j l_m),
 //    which k_bw_undeflate turns into +-c s dL/domega on the two d's.
-// `tpr` lanes per deflated row (where deflated rows are most of the level:
-// enough to reach lanes_target threads, at least ~8 roots per lane on
-// average); the lanes stride over the roots and combine by shuffles.  Every warp runs the same number of trips,
-// so the shuffles stay convergent.
-__global__ void __launch_bounds__(256) k_bw_defl(BArgs a, long long total_n) {
+// A warp classifies `rows` consecutive rows of the level, one per lane, and
+// shares its lanes among those that were deflated, tpr each (a power of
+// two), which stride over the roots and combine by shuffles.  The host picks
+// rows so that the warps just fill the GPU; the lanes then follow the
+// deflation of each place by themselves.  (With a lane count per level, the
+// few deflated rows of the low levels were left one thread each, a serial
+// loop of 125 loads; that bounded the pass: 34 us a level at n = 65,536.)
+__global__ void __launch_bounds__(256) k_bw_defl(BArgs a, long long total_n, int rows) {
     pdl_begin();
     if (halted(a.w.hdr)) {
         return;
     }
     const Ws &w = a.w;
-    const LevelCtl *ctl = &w.hdr->lvl[a.k];
-    const long long ndefl = a.level_rows - ctl->total_k;
-    const double kavg = (double)ctl->total_k / (double)(a.nodes > 0 ? a.nodes : 1);
-    // more lanes per row only where deflated rows are most of the level:
-    // below that, every extra lane mostly classifies rows that need nothing
-    int tpr = 1;
-    while (2 * ndefl > a.level_rows && tpr < 32 &&
-           (double)tpr * (double)ndefl < (double)a.lanes_target &&
-           8.0 * (double)(2 * tpr) <= kavg) {
-        tpr <<= 1;
-    }
-    const long long slots = ((total_n * tpr + 31) / 32) * 32;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < slots; t += stride) {
-        const long long x = t / tpr;
-        const int l = (int)(t % tpr);
-        double acc = 0.0;
-        bool out = false, small = false;
-        long long gs = 0, dst = 0;
-        double scale = 1.0;
+    const int lane = threadIdx.x & 31;
+    const long long warps = (long long)gridDim.x * (blockDim.x >> 5);
+    for (long long x0 = ((long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * rows;
+         x0 < total_n; x0 += warps * rows) {
+        // this lane's row
+        const long long x = x0 + lane;
+        int K = 0, q = 0;
+        bool small = false, mine = false;
+        long long gs = 0, po = 0;
+        double di = 0.0, fi = 0.0, li = 0.0, gfi = 0.0, gli = 0.0, scale = 0.0;
         int g, m, depth;
-        if (x < total_n && elem_node(a.F, a.k, x, &g, &gs, &m, &depth) && depth != 0) {
-            const long long po = (gs + g + 1) & ~1LL;
+        if (lane < rows && x < total_n && elem_node(a.F, a.k, x, &g, &gs, &m, &depth) &&
+            depth != 0) {
+            po = (gs + g + 1) & ~1LL;
             const int s = (int)(x - gs);
-            const int K = w.nK[g];
+            K = w.nK[g];
             const int Kz = w.nKz[g];
             const int ndz = m - Kz;
             if (s >= K) {
+                mine = true;
                 small = s < K + ndz;
-                const int q = small ? s - K : s - K - ndz;
-                double di, fi, li, gfi, gli, zp = 1.0;
+                q = small ? s - K : s - K - ndz;
                 if (small) {
                     di = w.zd[gs + q];
                     fi = w.zf[gs + q];
                     li = w.zl[gs + q];
                     gfi = w.bzf[gs + q];
                     gli = w.bzl[gs + q];
+                    // 1/N_j is in the scale of the Loewner weights, sqrt(rho)
+                    // z; the omega sum multiplies it by a weight of that scale
+                    scale = sqrt(w.nrho[g]);
                 } else {
                     const int act = w.gpos[gs + q];
                     const int p = lower_bound_int(w.pmap + po, K, w.gbase[gs + act]);
                     di = w.pd[po + p];
-                    zp = w.pw[po + p];
+                    scale = w.pw[po + p];
                     fi = w.af[gs + act];
                     li = w.al[gs + act];
                     gfi = w.bgf[gs + q];
                     gli = w.bgl[gs + q];
                 }
+            }
+        }
+        const unsigned who = __ballot_sync(kFull, mine);
+        const int nd = __popc(who);
+        int tpr = 32;
+        while (tpr > 1 && nd * tpr > 32) {
+            tpr >>= 1;
+        }
+        // group `grp` works on the warp's grp-th deflated row, held by lane src
+        const int grp = lane / tpr, l = lane & (tpr - 1);
+        const bool act = grp < nd;
+        int src = 0; // the set bit of `who` that has grp set bits below it
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            src += __popc(who & ((1u << (src + o)) - 1u)) <= grp ? o : 0;
+        }
+        src &= 31;
+        const int Kr = __shfl_sync(kFull, K, src);
+        const long long pr = __shfl_sync(kFull, po, src);
+        const bool sm = __shfl_sync(kFull, (int)small, src) != 0;
+        const double d = __shfl_sync(kFull, di, src);
+        const double f = __shfl_sync(kFull, fi, src), e = __shfl_sync(kFull, li, src);
+        const double gf = __shfl_sync(kFull, gfi, src), gl = __shfl_sync(kFull, gli, src);
+        const double sc = __shfl_sync(kFull, scale, src);
+        const long long dst = __shfl_sync(kFull, gs + q, src);
+        double acc = 0.0;
+        if (act) {
 #pragma unroll 4
-                for (int j = l; j < K; j += tpr) {
-                    const double r = brdc_rcp((di - __ldg(w.rdo + po + j)) - __ldg(w.rtau + po + j));
-                    const double tt = __ldg(w.bfr + po + j) * fi + __ldg(w.blr + po + j) * li -
-                                      gfi * __ldg(w.rfp + po + j) - gli * __ldg(w.rlp + po + j);
-                    acc += __ldg(w.rinvn + po + j) * r * (small ? tt : -tt * r);
-                }
-                out = true;
-                dst = gs + q;
-                // 1/N_j is in the scale of the Loewner weights, sqrt(rho) z;
-                // the omega sum multiplies it by a weight of the same scale
-                scale = small ? sqrt(w.nrho[g]) : zp;
+            for (int j = l; j < Kr; j += tpr) {
+                const double r = brdc_rcp((d - __ldg(w.rdo + pr + j)) - __ldg(w.rtau + pr + j));
+                const double tt = __ldg(w.bfr + pr + j) * f + __ldg(w.blr + pr + j) * e -
+                                  gf * __ldg(w.rfp + pr + j) - gl * __ldg(w.rlp + pr + j);
+                acc += __ldg(w.rinvn + pr + j) * r * (sm ? tt : -tt * r);
             }
         }
         acc = group_sum(acc, tpr);
-        if (out && l == 0) {
-            if (small) {
-                w.bzz[dst] = acc * scale;
-            } else {
-                w.bgw[dst] = scale * acc;
-            }
+        if (act && l == 0) {
+            (sm ? w.bzz : w.bgw)[dst] = sc * acc;
         }
     }
 }
@@ -509,18 +522,31 @@ __device__ inline bool bw_reverse_chain(const Ws &w, long long gs, int b0, int K
 }
 
 // ------------------------------------------------------------- undeflate
+// Entry i of a node's lists (active [0, Kz), then small-z) back to the child
+// row it came from, by way of its merged position (z = last row of the left
+// child / first row of the right child, over sqrt 2).
+__device__ __forceinline__ void bw_to_child(const Ws &w, long long gs, int m1, int Kz, int i,
+                                            bool top) {
+    const bool act = i < Kz;
+    const long long q = gs + (act ? i : i - Kz);
+    const int e = w.morig[gs + (act ? w.amap[q] : w.zmap[q])];
+    const double z = (act ? w.baz[q] : top ? 0.0 : w.bzz[q]) * 0.70710678118654752440;
+    const double f = act ? w.baf[q] : w.bzf[q], l = act ? w.bal[q] : w.bzl[q];
+    const long long x = gs + e;
+    w.bcd[x] = act ? w.bad[q] : w.bzd[q];
+    w.bcf[x] = e < m1 ? f : z;
+    w.bcl[x] = e < m1 ? z : l;
+}
+
 // One CTA per merge: pole and rotated-out cotangents back to the active
 // list, each Givens chain reversed (rows and z), active and small-z lists
-// back to merged positions, merged positions back to the two children
-// (z = last row of the left child / first row of the right child, over
-// sqrt 2), and dL/dE at the cut.
+// back to the two children, and dL/dE at the cut.
 template <int T>
 __global__ void __launch_bounds__(T) k_bw_undeflate(BArgs a) {
     pdl_begin();
     if (halted(a.w.hdr)) {
         return;
     }
-    __shared__ int iscan[32];
     __shared__ double red[32];
     const int g = blockIdx.x;
     const NodeGeom G = node_geom(a.F, a.k, g);
@@ -529,12 +555,9 @@ __global__ void __launch_bounds__(T) k_bw_undeflate(BArgs a) {
     const int m = G.m, m1 = G.m1;
     const int K = w.nK[g];
     const int Kz = w.nKz[g];
-    const int ndz = m - Kz;
     const bool top = (G.depth == 0);
-    const double isq2 = 0.70710678118654752440;
 
-    // poles -> active positions; rotated-out eigenvalues and rows by rank
-    // among the active positions with gmark set
+    // poles and rotated-out members -> active positions
     for (int i = threadIdx.x; i < K; i += T) {
         const long long o = gs + w.pmap[po + i];
         w.bad[o] = w.bpd[po + i];
@@ -542,23 +565,14 @@ __global__ void __launch_bounds__(T) k_bw_undeflate(BArgs a) {
         w.baf[o] = w.bpf[po + i];
         w.bal[o] = w.bpl[po + i];
     }
-    int carry = 0;
-    for (int base = 0; base < Kz; base += T) {
-        const int a0 = base + threadIdx.x;
-        const int mk = (a0 < Kz) ? w.gmark[gs + a0] : 0;
-        int tot;
-        const int ex = block_exscan<T>(mk, iscan, &tot);
-        if (mk) {
-            const int q = carry + ex;
-            const long long o = gs + a0;
-            w.bad[o] = w.bgd[gs + q];
-            // a rotated-out member's z is zero for every z, so its slot
-            // carries dL/domega to the chain reversal instead
-            w.baz[o] = top ? 0.0 : w.bgw[gs + q];
-            w.baf[o] = w.bgf[gs + q];
-            w.bal[o] = w.bgl[gs + q];
-        }
-        carry += tot;
+    for (int q = threadIdx.x; q < Kz - K; q += T) {
+        const long long o = gs + w.gpos[gs + q];
+        w.bad[o] = w.bgd[gs + q];
+        // a rotated-out member's z is zero for every z, so its slot carries
+        // dL/domega to the chain reversal instead
+        w.baz[o] = top ? 0.0 : w.bgw[gs + q];
+        w.baf[o] = w.bgf[gs + q];
+        w.bal[o] = w.bgl[gs + q];
     }
     __syncthreads();
 
@@ -573,35 +587,9 @@ __global__ void __launch_bounds__(T) k_bw_undeflate(BArgs a) {
     const double grho = block_sum<T>(kr, red);
     __syncthreads();
 
-    // active and small-z lists -> merged positions
-    for (int i = threadIdx.x; i < Kz; i += T) {
-        const long long p = gs + w.amap[gs + i];
-        w.bmd[p] = w.bad[gs + i];
-        w.bmz[p] = w.baz[gs + i];
-        w.bmf[p] = w.baf[gs + i];
-        w.bml[p] = w.bal[gs + i];
-    }
-    for (int q = threadIdx.x; q < ndz; q += T) {
-        const long long p = gs + w.zmap[gs + q];
-        w.bmd[p] = w.bzd[gs + q];
-        w.bmz[p] = top ? 0.0 : w.bzz[gs + q];
-        w.bmf[p] = w.bzf[gs + q];
-        w.bml[p] = w.bzl[gs + q];
-    }
-    __syncthreads();
-
-    // merged positions -> children
-    for (int p = threadIdx.x; p < m; p += T) {
-        const long long x = gs + w.morig[gs + p];
-        const int e = (int)(x - gs);
-        w.bcd[x] = w.bmd[gs + p];
-        if (e < m1) {
-            w.bcf[x] = w.bmf[gs + p];
-            w.bcl[x] = w.bmz[gs + p] * isq2;
-        } else {
-            w.bcf[x] = w.bmz[gs + p] * isq2;
-            w.bcl[x] = w.bml[gs + p];
-        }
+    // active and small-z lists -> the children's rows
+    for (int i = threadIdx.x; i < m; i += T) {
+        bw_to_child(w, gs, m1, Kz, i, top);
     }
     if (threadIdx.x == 0) {
         const long long cut = gs + m1 - 1;
@@ -610,7 +598,7 @@ __global__ void __launch_bounds__(T) k_bw_undeflate(BArgs a) {
 }
 
 // The same undeflation for the large merges near the top, where one CTA per
-// merge would stream tens of thousands of rows alone: five grid-wide passes
+// merge would stream tens of thousands of rows alone: four grid-wide passes
 // over the level's rows, each row one independent gather or scatter.  The
 // rotated-out slot q finds its active index through gpos, so no scan is
 // needed.
@@ -673,66 +661,18 @@ __global__ void __launch_bounds__(256) k_bw_ud_chains(BArgs a, long long total_n
     }
 }
 
-// active and small-z lists -> merged positions
-__global__ void __launch_bounds__(256) k_bw_ud_merged(BArgs a, long long total_n) {
-    pdl_begin();
-    if (halted(a.w.hdr)) {
-        return;
-    }
-    const Ws &w = a.w;
-    for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total_n;
-         x += (long long)gridDim.x * blockDim.x) {
-        int g, m, depth;
-        long long gs;
-        if (!elem_node(a.F, a.k, x, &g, &gs, &m, &depth)) {
-            continue;
-        }
-        const int s = (int)(x - gs);
-        const int Kz = w.nKz[g];
-        if (s < Kz) {
-            const long long p = gs + w.amap[gs + s];
-            w.bmd[p] = w.bad[gs + s];
-            w.bmz[p] = w.baz[gs + s];
-            w.bmf[p] = w.baf[gs + s];
-            w.bml[p] = w.bal[gs + s];
-        } else {
-            const int q = s - Kz;
-            const long long p = gs + w.zmap[gs + q];
-            w.bmd[p] = w.bzd[gs + q];
-            w.bmz[p] = depth == 0 ? 0.0 : w.bzz[gs + q];
-            w.bmf[p] = w.bzf[gs + q];
-            w.bml[p] = w.bzl[gs + q];
-        }
-    }
-}
-
-// merged positions -> children (z = last row of the left child / first row
-// of the right child, over sqrt 2)
+// active and small-z lists -> the children's rows
 __global__ void __launch_bounds__(256) k_bw_ud_children(BArgs a, long long total_n) {
     pdl_begin();
     if (halted(a.w.hdr)) {
         return;
     }
-    const Ws &w = a.w;
-    const double isq2 = 0.70710678118654752440;
     for (long long x = (long long)blockIdx.x * blockDim.x + threadIdx.x; x < total_n;
          x += (long long)gridDim.x * blockDim.x) {
         int g, m, depth;
         long long gs;
-        if (!elem_node(a.F, a.k, x, &g, &gs, &m, &depth)) {
-            continue;
-        }
-        const int p = (int)(x - gs);
-        const int m1 = m >> 1;
-        const long long xc = gs + w.morig[gs + p];
-        const int e = (int)(xc - gs);
-        w.bcd[xc] = w.bmd[x];
-        if (e < m1) {
-            w.bcf[xc] = w.bmf[x];
-            w.bcl[xc] = w.bmz[x] * isq2;
-        } else {
-            w.bcf[xc] = w.bmz[x] * isq2;
-            w.bcl[xc] = w.bml[x];
+        if (elem_node(a.F, a.k, x, &g, &gs, &m, &depth)) {
+            bw_to_child(a.w, gs, m >> 1, a.w.nKz[g], (int)(x - gs), depth == 0);
         }
     }
 }

@@ -245,8 +245,7 @@ const SlotDesc kSlots[] = {
     // adjoint
     SD(bcd, CN_NT, false, true), SD(bcf, CN_NT, false, true), SD(bcl, CN_NT, false, true),
     SD(bnd, CN_NT, false, true), SD(bnf, CN_NT, false, true), SD(bnl, CN_NT, false, true),
-    SD(bmd, CN_NT, false, true), SD(bmz, CN_NT, false, true), SD(bmf, CN_NT, false, true),
-    SD(bml, CN_NT, false, true), SD(bad, CN_NT, false, true), SD(baz, CN_NT, false, true),
+    SD(bad, CN_NT, false, true), SD(baz, CN_NT, false, true),
     SD(baf, CN_NT, false, true), SD(bal, CN_NT, false, true), SD(bzd, CN_NT, false, true),
     SD(bzf, CN_NT, false, true), SD(bzl, CN_NT, false, true), SD(bgd, CN_NT, false, true),
     SD(bgf, CN_NT, false, true), SD(bgl, CN_NT, false, true),
@@ -1961,7 +1960,13 @@ brdc_status run_backward(brdc_handle h, const HostForest &hf, const Layout &L,
     double *out[3] = {w.bcd, w.bcf, w.bcl};
     // k_bw_roots and k_bw_poles: 64 registers or fewer, four blocks per SM
     const int wgrid = h->sm_count * 4;
-    long long dgrid = (4 * nt + 255) / 256;
+    // k_bw_defl: rows a warp classifies, so that four blocks per SM (64
+    // registers) hold the level, 32 at most
+    int drows = 1;
+    while (drows < 32 && (long long)drows * h->sm_count * 32 < nt) {
+        drows *= 2;
+    }
+    long long dgrid = (nt + 8 * drows - 1) / (8 * drows);
     dgrid = std::max<long long>(1, std::min<long long>(dgrid, (long long)h->sm_count * 16));
     for (int k = hf.max_levels - 1; k >= 0; --k) {
         Ws wl = w;
@@ -1983,19 +1988,16 @@ brdc_status run_backward(brdc_handle h, const HostForest &hf, const Layout &L,
         b.k = k;
         b.nodes = hf.level_nodes[k];
         b.level_rows = hf.level_rows[k];
-        b.lanes_target = h->lanes_target;
         launch_pdl(k_bw_unplace, eg, 256, s, b, nt);
         launch_pdl(k_bw_roots, wgrid, kSweepThreads, s, b);
         launch_pdl(k_bw_poles, wgrid, kSweepThreads, s, b);
         if (k + 1 < hf.max_levels || hf.B > 1) {
-            // up to 4 lanes per row (the kernel picks); surplus blocks exit
-            launch_pdl(k_bw_defl, dgrid, 256, s, b, nt);
+            launch_pdl(k_bw_defl, dgrid, 256, s, b, nt, drows);
         }
         if (hf.level_mmax[k] >= 2 * kDeflEPT * 1024) {
             // large merges: grid-wide passes instead of one CTA per merge
             launch_pdl(k_bw_ud_active, eg, 256, s, b, nt);
             launch_pdl(k_bw_ud_chains, eg, 256, s, b, nt);
-            launch_pdl(k_bw_ud_merged, eg, 256, s, b, nt);
             launch_pdl(k_bw_ud_children, eg, 256, s, b, nt);
             launch_pdl(k_bw_ud_rho, std::max(1, std::min(b.nodes / 8 + 1, h->sm_count * 8)), 256, s, b);
         } else {

@@ -182,7 +182,6 @@ struct Ws {
     long long *f_norm;           // per instance: bits of max(|D|, |E|) (>= 0)
     // adjoint (present when the workspace keeps checkpoints)
     double *bcd, *bcf, *bcl, *bnd, *bnf, *bnl;   // cotangents, ping-pong
-    double *bmd, *bmz, *bmf, *bml;               // at merged positions
     double *bad, *baz, *baf, *bal;               // at active positions
     double *bzd, *bzf, *bzl, *bgd, *bgf, *bgl;   // deflated lists
     double *blam, *bfr, *blr;                    // per root (padded)
