@@ -850,6 +850,11 @@ brdc_status run_forest(brdc_handle h, const HostForest &hf, const Layout &L,
         static_assert(sizeof(PlanAllArgs) <= 4096, "kernel parameters of k_plan_all");
         PlanAllArgs P{};
         P.base = a;
+        // a root's or pole's share of an adjoint pass ends in a serial part
+        // of one lane, so a quarter of the forward's lanes are taken (step
+        // of normal 65,536: 1291 us at the forward's lanes, 1199 at a
+        // quarter, 1263 at an eighth; uniform 16,384 879, 797, 823)
+        P.base.lanes_target = std::max(1, h->lanes_target / 4);
         int cnt = 0;
         for (int k = 0; k < hf.max_levels && cnt < kPlanMaxLevels; ++k) {
             const bool sub_level = sub > 0 && k < fused;
@@ -1926,9 +1931,14 @@ void launch_undeflate(const BArgs &b, int grid, cudaStream_t s) {
     launch_pdl(k_bw_undeflate<T>, grid, T, s, b);
 }
 
-void launch_undeflate_sized(const BArgs &b, int mmax, cudaStream_t s) {
+void launch_undeflate_sized(const BArgs &b, int mmax, int sms, cudaStream_t s) {
+    // a thread per row while that is less than half a wave of threads (the
+    // passes are dependent loads: forward and backward of normal 4,096 507
+    // -> 488 us), else one per four rows at least (fit of 1024: 7.70 ms with
+    // a thread per row, 7.53 with a quarter)
     int t = 32;
-    while (t < 1024 && t * 4 < mmax) {
+    while (t < 1024 && t < mmax &&
+           (t * 4 < mmax || (long long)b.nodes * 2 * t <= (long long)sms * 1024)) {
         t <<= 1;
     }
     switch (t) {
@@ -1960,10 +1970,10 @@ brdc_status run_backward(brdc_handle h, const HostForest &hf, const Layout &L,
     double *out[3] = {w.bcd, w.bcf, w.bcl};
     // k_bw_roots and k_bw_poles: 64 registers or fewer, four blocks per SM
     const int wgrid = h->sm_count * 4;
-    // k_bw_defl: rows a warp classifies, so that four blocks per SM (64
-    // registers) hold the level, 32 at most
+    // k_bw_defl: rows a warp classifies, so that two waves of warps (64
+    // registers a thread) hold the level, 32 at most
     int drows = 1;
-    while (drows < 32 && (long long)drows * h->sm_count * 32 < nt) {
+    while (drows < 32 && (long long)drows * h->sm_count * 64 < nt) {
         drows *= 2;
     }
     long long dgrid = (nt + 8 * drows - 1) / (8 * drows);
@@ -2001,7 +2011,7 @@ brdc_status run_backward(brdc_handle h, const HostForest &hf, const Layout &L,
             launch_pdl(k_bw_ud_children, eg, 256, s, b, nt);
             launch_pdl(k_bw_ud_rho, std::max(1, std::min(b.nodes / 8 + 1, h->sm_count * 8)), 256, s, b);
         } else {
-            launch_undeflate_sized(b, hf.level_mmax[k], s);
+            launch_undeflate_sized(b, hf.level_mmax[k], h->sm_count, s);
         }
         BRDC_CUDA(h, "brdc.bw.level", cudaGetLastError());
         std::swap(par[0], out[0]);
