@@ -1514,6 +1514,17 @@ __device__ inline SecTot secular_shared(const SecRoot &st, const double *pd, con
     return sec_total(sum);
 }
 
+// A root's sums over its lanes with the bound of sec_bound (K poles).
+__device__ inline void sums_reduce_shared(SecTot &sum, int tpr, int K) {
+    for (int o = tpr >> 1; o > 0; o >>= 1) {
+        sum.sum += __shfl_xor_sync(0xffffffffu, sum.sum, o);
+        sum.mag += __shfl_xor_sync(0xffffffffu, sum.mag, o);
+        sum.dpsi += __shfl_xor_sync(0xffffffffu, sum.dpsi, o);
+        sum.dphi += __shfl_xor_sync(0xffffffffu, sum.dphi, o);
+    }
+    sec_bound(sum, K >> (31 - __clz(tpr)));
+}
+
 __device__ inline void sums_reduce(SecTot &sum, int tpr) {
     for (int o = tpr >> 1; o > 0; o >>= 1) {
         SecTot other;

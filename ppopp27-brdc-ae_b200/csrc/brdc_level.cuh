@@ -383,7 +383,7 @@ __device__ void level_roots(LvlSmem &S, cooperative_groups::cluster_group &cl, c
                 if (live) {
                     sum = secular_shared(st, S.pd, S.pz, K, l2, tp, r < K - 2 ? r : K - 2, r + 1);
                 }
-                sums_reduce(sum, tp);
+                sums_reduce_shared(sum, tp, K);
                 if (live) {
                     sec_after_sweep(st, sum, eps, max_iter);
                 }

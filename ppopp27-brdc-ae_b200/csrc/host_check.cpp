@@ -40,6 +40,7 @@ extern "C" int brdc_host_secular_root_any(int K, const double *d, const double *
             }
         }
         ++sweeps;
+        brdc::sec_bound(t[0], (K + lanes - 1) / lanes);
         brdc::sec_after_sweep(r, t[0], DBL_EPSILON);
     }
     *org = r.org;
