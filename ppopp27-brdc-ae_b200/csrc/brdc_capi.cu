@@ -675,6 +675,7 @@ int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, boo
     // costs a level 4 us.)
     const bool big = mmax > (hf.B > 1 ? kBoxMinK : kLvlMaxK);
     a.big_k = big ? kBoxMinK : kLvlMaxK;
+    a.keep = ckpt ? 1 : 0;
     a.plan_inline = big && a.nodes <= kLvlThreads ? 1 : 0;
     cudaLaunchAttribute at[2];
     cudaLaunchConfig_t cfg = cluster_config((unsigned)(a.nodes * C), C, s, at);
@@ -703,7 +704,6 @@ int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, boo
         mark(h, 5 + 4 * k);
         mark(h, 6 + 4 * k);
     }
-    (void)ckpt; // the adjoint's full plan of this level comes with run_forest's last launch
     return n;
 }
 

@@ -45,6 +45,7 @@ struct KArgs {
     long long level_rows; // rows of the instances that merge at this level
     int plan_inline;    // the last deflation CTA writes the level plan (else k_plan)
     int lanes_target;   // threads the root sweeps aim to keep busy
+    int keep;           // the workspace keeps checkpoints: write what the adjoint reads
     int big_k;          // > 0: the plan and the placement serve only nodes with
                         // K > big_k (k_level finished the others)
 };

@@ -40,11 +40,23 @@ constexpr int kLvlMergeChunk = 4096; // merged positions per chunk of the merge 
 // (uniform 65,536, level 7: 53 -> 48 us); 8192 gained nothing more, 16384
 // lost.
 constexpr int kLvlSoloDeflRows = 4096;
+// Merges of at most this many rows are merged and deflated by every CTA of
+// their cluster, each for itself in shared memory (level_merge_local): no
+// merged list goes to L2 and back, and no cluster barrier is needed before
+// the roots.  One chunk of kDeflEPT rows a thread, and what `stage` holds.
+// Measured on B200 (normal 4,096, whose levels above the subtree have 256 to
+// 4096 rows): merge and deflation of a level 9 -> 5-7 us, the solve 238 ->
+// 227.
+constexpr int kLvlLocalRows = 2048;
+static_assert(kLvlLocalRows == kDeflEPT * kLvlThreads && 4 * kLvlLocalRows <= 2 * kLvlSamples &&
+                  3 * kLvlLocalRows <= 7 * kLvlMaxK && kLvlMaxK <= 2 * kLvlThreads,
+              "local merges");
 
 struct LvlSmem {
     double pd[kLvlMaxK], pz[kLvlMaxK], pf[kLvlMaxK], pl[kLvlMaxK], pw[kLvlMaxK];
     double rdo[kLvlMaxK], rtau[kLvlMaxK];
     double stage[2 * kLvlSamples];       // staged sorted lists of the placement
+    int amap[kLvlMaxK], gmark[kLvlMaxK], gbase[kLvlMaxK]; // active list (level_poles)
     double red[32];
     int iscan[32];
     double s_val;                        // cluster exchange
@@ -304,6 +316,219 @@ __device__ void level_place_merge(const KArgs &a, const Ws &w, LvlSmem &S, doubl
     }
 }
 
+// The merged list of a node of at most kLvlLocalRows rows, by the CTA alone,
+// and its small-z test: the merge path over both children in shared memory,
+// then defl_compact_active's compaction, whose survivors stay in pd, pz, pf,
+// pl, amap and gmark of this CTA (unless they are more than kLvlMaxK: then
+// the CTAs write the merged list in shares, for the general path).  Of the
+// small-z rows, and with `keep` of what the adjoint reads, each CTA writes
+// the merged positions [e0, e1).  Returns the survivors; *tol_out the
+// tolerance.
+template <int T>
+__device__ int level_merge_local(LvlSmem &S, double *buf, const Ws &w, long long gs, int m1, int m,
+                                 int e0, int e1, double rho, double maxd, bool keep,
+                                 double *tol_out) {
+    constexpr int EPT = kDeflEPT;
+    const int x = threadIdx.x, m2 = m - m1;
+    double *bd = buf, *bf = buf + kLvlLocalRows, *bl = buf + 2 * kLvlLocalRows;
+    double *md = S.stage, *mz = md + kLvlLocalRows, *mf = mz + kLvlLocalRows,
+           *ml = mf + kLvlLocalRows;
+    for (int u = x; u < m; u += T) {
+        bd[u] = w.cd[gs + u];
+        bf[u] = w.cf[gs + u];
+        bl[u] = w.cl[gs + u];
+    }
+    __syncthreads();
+    double lz = 0.0;
+    for (int k = x; k < m; k += T) {
+        int lo = max(0, k - m2), hi = min(k, m1);
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (bd[mid] <= bd[m1 + k - mid - 1]) {
+                lo = mid + 1;
+            } else {
+                hi = mid;
+            }
+        }
+        const int i = lo, j = k - lo;
+        const bool left = i < m1 && (j >= m2 || bd[i] <= bd[m1 + j]);
+        const int u = left ? i : m1 + j;
+        const double z = (left ? bl[u] : bf[u]) / kSqrt2;
+        md[k] = bd[u];
+        mz[k] = z;
+        mf[k] = left ? bf[u] : 0.0;
+        ml[k] = left ? 0.0 : bl[u];
+        lz = fmax(lz, fabs(z));
+        if (keep && k >= e0 && k < e1) {
+            w.md[gs + k] = bd[u];
+            w.mz[gs + k] = z;
+            w.morig[gs + k] = u;
+        }
+    }
+    const double tol = kDeflTolScale * DBL_EPSILON * fmax(maxd, block_max<T>(lz, S.red));
+    *tol_out = tol;
+    // block_max ends with every thread past the merge: pd .. take the
+    // survivors where the children lay
+    __syncthreads();
+    const int lane = x & 31, wbase = (x >> 5) * (EPT * 32);
+    const unsigned lt = (1u << lane) - 1u;
+    bool fl[EPT];
+    unsigned bal[EPT];
+    int wcnt = 0;
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) {
+        const int idx = wbase + 32 * q + lane;
+        fl[q] = idx < m && fabs(rho * mz[idx]) > tol;
+        bal[q] = __ballot_sync(kFull, fl[q]);
+        wcnt += __popc(bal[q]);
+    }
+    int Kz;
+    int before = defl_warp_prefix<T>(wcnt, S.iscan, &Kz);
+    const bool fits = Kz <= kLvlMaxK;
+#pragma unroll
+    for (int q = 0; q < EPT; ++q) {
+        const int idx = wbase + 32 * q + lane;
+        if (idx < m) {
+            const int na = before + __popc(bal[q] & lt); // survivors before this row
+            if (!fits) {
+                if (idx >= e0 && idx < e1) {
+                    w.md[gs + idx] = md[idx];
+                    w.mz[gs + idx] = mz[idx];
+                    w.mf[gs + idx] = mf[idx];
+                    w.ml[gs + idx] = ml[idx];
+                }
+            } else if (fl[q]) {
+                S.pd[na] = md[idx];
+                S.pz[na] = mz[idx];
+                S.pf[na] = mf[idx];
+                S.pl[na] = ml[idx];
+                S.amap[na] = idx;
+                S.gmark[na] = 0;
+            } else if (idx >= e0 && idx < e1) {
+                const long long o = gs + idx - na;
+                w.zd[o] = md[idx];
+                w.zf[o] = mf[idx];
+                w.zl[o] = ml[idx];
+                if (keep) {
+                    w.zmap[o] = idx;
+                }
+            }
+        }
+        before += __popc(bal[q]);
+    }
+    __syncthreads();
+    return Kz;
+}
+
+// The active list that the cluster wrote, into this CTA's shared memory.
+template <int T>
+__device__ void level_load_active(LvlSmem &S, const Ws &w, long long gs, int Kz, bool keep) {
+    for (int i = threadIdx.x; i < Kz; i += T) {
+        S.pd[i] = __ldcg(w.ad + gs + i);
+        S.pz[i] = __ldcg(w.az + gs + i);
+        S.pf[i] = __ldcg(w.af + gs + i);
+        S.pl[i] = __ldcg(w.al + gs + i);
+        S.amap[i] = keep ? __ldcg(w.amap + gs + i) : 0;
+        S.gmark[i] = 0;
+    }
+    __syncthreads();
+}
+
+// Close-pole chains and the poles of an active list of Kz <= kLvlMaxK entries
+// in this CTA's pd .. gmark: every CTA of the cluster does them for itself,
+// CTA 0 (`writer`) writes the lists.  pd, pz, pf and pl end as the K poles;
+// returns sum z^2 over them.
+template <int T>
+__device__ double level_poles(LvlSmem &S, const Ws &w, long long gs, long long po, int Kz,
+                              double tol, bool writer, bool keep, int big_k, int *K_out) {
+    const int x = threadIdx.x;
+    // the walk on the shared lists; the rotations' own record is CTA 0's
+    Ws v = w;
+    v.ad = S.pd;
+    v.az = S.pz;
+    v.af = S.pf;
+    v.al = S.pl;
+    v.gmark = S.gmark;
+    v.gbase = S.gbase;
+    v.gc = writer ? w.gc + gs : S.stage;
+    v.gs = writer ? w.gs + gs : S.stage + kLvlMaxK;
+    v.gr = writer ? w.gr + gs : S.stage + 2 * kLvlMaxK;
+    const bool rot = __syncthreads_or(defl_close_walk<T>(v, 0, Kz, tol, 0, Kz));
+    if (writer && keep) {
+        for (int i = x; i < Kz; i += T) {
+            w.ad[gs + i] = S.pd[i];
+            w.az[gs + i] = S.pz[i];
+            w.af[gs + i] = S.pf[i];
+            w.al[gs + i] = S.pl[i];
+            w.amap[gs + i] = S.amap[i];
+            w.gmark[gs + i] = S.gmark[i];
+            w.gbase[gs + i] = S.gbase[i];
+        }
+    }
+    int K = Kz;
+    if (rot) {
+        // poles closed up in place, rotated-out members to their list
+        double vd[2], vz[2], vf[2], vl[2];
+        bool pole[2], in[2];
+        int np[2];
+        int carry = 0;
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = x + q * T;
+            in[q] = i < Kz;
+            pole[q] = in[q] && S.gmark[i] == 0;
+            int tot;
+            np[q] = carry + block_exscan<T>(pole[q] ? 1 : 0, S.iscan, &tot);
+            carry += tot;
+            if (in[q]) {
+                vd[q] = S.pd[i];
+                vz[q] = S.pz[i];
+                vf[q] = S.pf[i];
+                vl[q] = S.pl[i];
+            }
+        }
+        K = carry;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int i = x + q * T;
+            if (pole[q]) {
+                S.pd[np[q]] = vd[q];
+                S.pz[np[q]] = vz[q];
+                S.pf[np[q]] = vf[q];
+                S.pl[np[q]] = vl[q];
+                if (writer) {
+                    w.pmap[po + np[q]] = i;
+                }
+            } else if (in[q] && writer) {
+                const long long o = gs + i - np[q];
+                w.gd[o] = vd[q];
+                w.gf[o] = vf[q];
+                w.gl[o] = vl[q];
+                w.gpos[o] = i;
+            }
+        }
+        __syncthreads();
+    }
+    double zn = 0.0;
+    const bool out = writer && (keep || K > big_k);
+    for (int i = x; i < K; i += T) {
+        const double z = S.pz[i];
+        zn += z * z;
+        if (out) {
+            w.pd[po + i] = S.pd[i];
+            w.pz[po + i] = z;
+            w.pf[po + i] = S.pf[i];
+            w.pl[po + i] = S.pl[i];
+            if (!rot) {
+                w.pmap[po + i] = i;
+            }
+        }
+    }
+    *K_out = K;
+    return block_sum<T>(zn, S.red);
+}
+
 // Roots, Loewner weights and boundary rows of one node with 1 <= K <=
 // kLvlMaxK poles, by all C CTAs of its cluster: CTA r takes the roots (and
 // poles) [r P, (r+1) P), P = ceil(K / C), and gathers the others' from their
@@ -312,7 +537,8 @@ __device__ void level_place_merge(const KArgs &a, const Ws &w, LvlSmem &S, doubl
 // with a cluster barrier, after which no CTA reads a peer's shared memory.
 template <int T>
 __device__ void level_roots(LvlSmem &S, cooperative_groups::cluster_group &cl, const KArgs &a,
-                            const NodeGeom &G, int K, double rho, double zn, int C, int rank) {
+                            const NodeGeom &G, int K, double rho, double zn, int C, int rank,
+                            bool staged) {
     const Ws &w = a.w;
     const long long po = G.poff;
     const int x = threadIdx.x, lane = x & 31;
@@ -326,8 +552,8 @@ __device__ void level_roots(LvlSmem &S, cooperative_groups::cluster_group &cl, c
     // cluster barrier), hence the proxy fence before the copies.  A wait
     // past the handle's limit is followed by a bounded drain, so the block
     // never moves on with copies in flight; only a failed drain records an
-    // error.
-    {
+    // error.  (`staged`: level_poles left them there.)
+    if (!staged) {
         const unsigned bytes = (unsigned)(((K + 1) & ~1) * sizeof(double));
         if (x == 0) {
             mbar_init(&S.bar, 1);
@@ -566,114 +792,134 @@ __global__ void __launch_bounds__(T, 1) k_level(KArgs a) {
     // (left wins ties), as k_merge, by the merge path; max|z| on the way
     const int SE = (m + C - 1) / C;
     const int e0 = min(m, rank * SE), e1 = min(m, e0 + SE);
-    double lz = level_merge<T>(w, gs, m1, m, e0, e1,
-                               reinterpret_cast<double *>(lvl_raw + offsetof(LvlSmem, pd)),
-                               S.iscan, S.msplit);
-    lz = block_max<T>(lz, S.red);
-    if (x == 0) {
-        S.s_val = lz;
+    double *const buf = reinterpret_cast<double *>(lvl_raw + offsetof(LvlSmem, pd));
+    const bool keep = a.keep != 0;
+    double tol;
+    int K = 0, Kz = 0;
+    double zn = 0.0;
+    bool local = false; // this CTA's shared memory holds the poles
+    if (m <= kLvlLocalRows) {
+        Kz = level_merge_local<T>(S, buf, w, gs, m1, m, e0, e1, rho, maxd, keep, &tol);
+        local = Kz <= kLvlMaxK;
+        if (!local) {
+            cl.sync();
+        }
+    } else {
+        double lz = level_merge<T>(w, gs, m1, m, e0, e1, buf, S.iscan, S.msplit);
+        lz = block_max<T>(lz, S.red);
+        if (x == 0) {
+            S.s_val = lz;
+        }
+        // the cluster barrier releases and acquires at cluster scope, which
+        // orders the global writes of every phase for the peer CTAs
+        cl.sync();
+        double maxz = 0.0;
+        for (int r = 0; r < C; ++r) {
+            maxz = fmax(maxz, *cl.map_shared_rank(&S.s_val, r));
+        }
+        tol = kDeflTolScale * DBL_EPSILON * fmax(maxd, maxz);
     }
-    // the cluster barrier releases and acquires at cluster scope, which
-    // orders the global writes of every phase for the peer CTAs
-    cl.sync();
-    double maxz = 0.0;
-    for (int r = 0; r < C; ++r) {
-        maxz = fmax(maxz, *cl.map_shared_rank(&S.s_val, r));
-    }
-    const double tol = kDeflTolScale * DBL_EPSILON * fmax(maxd, maxz);
 
     // ------------------------------------------------ deflation
-    int K, Kz;
-    double zn;
-    if (C == 1) {
-        Kz = defl_compact_active<T>(w, gs, 0, m, rho, tol, 0, 0, S.iscan);
-        __syncthreads();
-        defl_close_walk<T>(w, gs, Kz, tol, 0, Kz);
-        __syncthreads();
-        zn = defl_compact_poles<T>(w, gs, G.poff, 0, Kz, 0, 0, S.iscan, &K);
-        zn = block_sum<T>(zn, S.red);
-    } else if (m <= kLvlSoloDeflRows || m <= ((m + C - 1) / C + chunk - 1) / chunk * chunk) {
-        // a small merge (or one that lies in CTA 0's deflation slice alone,
-        // the slices being whole chunks): CTA 0 deflates it as one CTA per
-        // node does, with no counts to exchange, and its peers wait at one
-        // cluster barrier
-        if (rank == 0) {
-            Kz = defl_compact_active<T>(w, gs, 0, m, rho, tol, 0, 0, S.iscan);
-            __syncthreads();
-            defl_close_walk<T>(w, gs, Kz, tol, 0, Kz);
-            __syncthreads();
-            zn = defl_compact_poles<T>(w, gs, G.poff, 0, Kz, 0, 0, S.iscan, &K);
-            zn = block_sum<T>(zn, S.red);
-            if (x == 0) {
-                S.s_cnt = K;
-                S.s_kz = Kz;
-                S.s_zn = zn;
-            }
-        }
-        cl.sync();
-        K = *cl.map_shared_rank(&S.s_cnt, 0);
-        Kz = *cl.map_shared_rank(&S.s_kz, 0);
-        zn = *cl.map_shared_rank(&S.s_zn, 0);
-    } else {
+    if (!local) {
+        // the active list: a small merge (or one that lies in CTA 0's
+        // deflation slice alone, the slices being whole chunks) by CTA 0 as
+        // one CTA per node does, its peers waiting at one cluster barrier
         const int SD = ((m + C - 1) / C + chunk - 1) / chunk * chunk;
-        const int r0 = min(m, rank * SD), r1 = min(m, r0 + SD);
-        const int na = defl_count_active<T>(w, gs, r0, r1, rho, tol, S.iscan);
-        if (x == 0) {
-            S.s_cnt = na;
-        }
-        cl.sync();
-        int off_a = 0;
-        Kz = 0;
-        for (int r = 0; r < C; ++r) {
-            const int cn = *cl.map_shared_rank(&S.s_cnt, r);
-            off_a += r < rank ? cn : 0;
-            Kz += cn;
-        }
-        defl_compact_active<T>(w, gs, r0, r1, rho, tol, off_a, r0 - off_a, S.iscan);
-        cl.sync();
-        const int A = (Kz + C - 1) / C;
-        const int rot = __syncthreads_or(
-            defl_close_walk<T>(w, gs, Kz, tol, min(Kz, rank * A), min(Kz, rank * A + A)));
-        if (x == 0) {
-            S.s_rot = rot;
-        }
-        cl.sync();
-        bool any_rot = false;
-        for (int r = 0; r < C; ++r) {
-            any_rot |= *cl.map_shared_rank(&S.s_rot, r) != 0;
-        }
-        const int S2 = ((Kz + C - 1) / C + chunk - 1) / chunk * chunk;
-        const int q0 = min(Kz, rank * S2), q1 = min(Kz, q0 + S2);
-        int off_p = q0;
-        K = Kz;
-        if (any_rot) {
-            // some entries were rotated out: count the poles of every
-            // slice (with none, every active entry is a pole)
-            const int np = defl_count_poles<T>(w, gs, q0, q1, S.iscan);
-            if (x == 0) {
-                S.s_cnt = np;
+        const bool solo = C == 1 || m <= kLvlSoloDeflRows || m <= SD;
+        if (solo) {
+            if (rank == 0) {
+                Kz = defl_compact_active<T>(w, gs, 0, m, rho, tol, 0, 0, S.iscan);
+                if (x == 0) {
+                    S.s_kz = Kz;
+                }
             }
             cl.sync();
-            off_p = 0;
-            K = 0;
+            Kz = *cl.map_shared_rank(&S.s_kz, 0);
+        } else {
+            const int r0 = min(m, rank * SD), r1 = min(m, r0 + SD);
+            const int na = defl_count_active<T>(w, gs, r0, r1, rho, tol, S.iscan);
+            if (x == 0) {
+                S.s_cnt = na;
+            }
+            cl.sync();
+            int off_a = 0;
+            Kz = 0;
             for (int r = 0; r < C; ++r) {
                 const int cn = *cl.map_shared_rank(&S.s_cnt, r);
-                off_p += r < rank ? cn : 0;
-                K += cn;
+                off_a += r < rank ? cn : 0;
+                Kz += cn;
+            }
+            defl_compact_active<T>(w, gs, r0, r1, rho, tol, off_a, r0 - off_a, S.iscan);
+            cl.sync();
+        }
+        if (Kz <= kLvlMaxK) {
+            // few poles: every CTA takes the list and goes on for itself,
+            // with no more counts to exchange
+            level_load_active<T>(S, w, gs, Kz, keep);
+            local = true;
+        } else if (solo) {
+            if (rank == 0) {
+                defl_close_walk<T>(w, gs, Kz, tol, 0, Kz);
+                __syncthreads();
+                zn = defl_compact_poles<T>(w, gs, G.poff, 0, Kz, 0, 0, S.iscan, &K);
+                zn = block_sum<T>(zn, S.red);
+                if (x == 0) {
+                    S.s_cnt = K;
+                    S.s_zn = zn;
+                }
+            }
+            cl.sync();
+            K = *cl.map_shared_rank(&S.s_cnt, 0);
+            zn = *cl.map_shared_rank(&S.s_zn, 0);
+        } else {
+            const int A = (Kz + C - 1) / C;
+            const int rot = __syncthreads_or(
+                defl_close_walk<T>(w, gs, Kz, tol, min(Kz, rank * A), min(Kz, rank * A + A)));
+            if (x == 0) {
+                S.s_rot = rot;
+            }
+            cl.sync();
+            bool any_rot = false;
+            for (int r = 0; r < C; ++r) {
+                any_rot |= *cl.map_shared_rank(&S.s_rot, r) != 0;
+            }
+            const int S2 = ((Kz + C - 1) / C + chunk - 1) / chunk * chunk;
+            const int q0 = min(Kz, rank * S2), q1 = min(Kz, q0 + S2);
+            int off_p = q0;
+            K = Kz;
+            if (any_rot) {
+                // some entries were rotated out: count the poles of every
+                // slice (with none, every active entry is a pole)
+                const int np = defl_count_poles<T>(w, gs, q0, q1, S.iscan);
+                if (x == 0) {
+                    S.s_cnt = np;
+                }
+                cl.sync();
+                off_p = 0;
+                K = 0;
+                for (int r = 0; r < C; ++r) {
+                    const int cn = *cl.map_shared_rank(&S.s_cnt, r);
+                    off_p += r < rank ? cn : 0;
+                    K += cn;
+                }
+            }
+            int end_p;
+            double zp = defl_compact_poles<T>(w, gs, G.poff, q0, q1, off_p, q0 - off_p, S.iscan,
+                                              &end_p);
+            zp = block_sum<T>(zp, S.red);
+            if (x == 0) {
+                S.s_val = zp;
+            }
+            cl.sync();
+            zn = 0.0;
+            for (int r = 0; r < C; ++r) {
+                zn += *cl.map_shared_rank(&S.s_val, r);
             }
         }
-        int end_p;
-        double zp = defl_compact_poles<T>(w, gs, G.poff, q0, q1, off_p, q0 - off_p, S.iscan,
-                                          &end_p);
-        zp = block_sum<T>(zp, S.red);
-        if (x == 0) {
-            S.s_val = zp;
-        }
-        cl.sync();
-        zn = 0.0;
-        for (int r = 0; r < C; ++r) {
-            zn += *cl.map_shared_rank(&S.s_val, r);
-        }
+    }
+    if (local) {
+        zn = level_poles<T>(S, w, gs, G.poff, Kz, tol, rank == 0, keep, a.big_k, &K);
     }
     if (rank == 0 && x == 0) {
         w.nK[g] = K;
@@ -703,7 +949,7 @@ __global__ void __launch_bounds__(T, 1) k_level(KArgs a) {
 
     // ------------------------------------------------ roots
     if (K > 0) {
-        level_roots<T>(S, cl, a, G, K, rho, zn, C, rank);
+        level_roots<T>(S, cl, a, G, K, rho, zn, C, rank, local);
     }
     cl.sync();
 
