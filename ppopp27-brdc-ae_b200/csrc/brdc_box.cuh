@@ -17,12 +17,12 @@
 // is narrow.  A box whose far part would be less than half of the poles
 // (clusters straddled by its interval) sums all of them directly.  The last
 // root, whose bracket leaves the poles' range, is summed directly by a whole
-// warp.
+// block.
 //
 // Bound: FP64 arithmetic.  Measured on B200 against sweeps over all poles
 // (k_sweeps, which still serves levels with the fused kernel off): Toeplitz
-// 16,384 2.31 -> 1.26 ms, 65,536 20.3 -> 5.0 ms, the mixed batch of 4096
-// matrices 66 -> 38 ms; largest error of Toeplitz 16,384 against its closed
+// 16,384 2.31 -> 1.05 ms, 65,536 20.3 -> 3.6 ms, the mixed batch of 4096
+// matrices 66 -> 37 ms; largest error of Toeplitz 16,384 against its closed
 // form 1.3e-16 -> 0.9e-16 of the norm.
 #pragma once
 
@@ -31,8 +31,12 @@
 namespace brdc {
 
 constexpr int kBoxP = 24;        // Chebyshev points of an interpolant
-constexpr int kBoxNodes = kBoxP / (kSweepThreads / 32); // points a warp sums
-static_assert(kBoxNodes * (kSweepThreads / 32) == kBoxP, "points per warp");
+// Points a warp sums over its share of the poles: 6 points keep a pole's two
+// loads hidden behind 42 FP64 instructions; the block's 8 warps are 4 groups
+// of points by 2 halves of the poles.
+constexpr int kBoxNodes = 6;
+constexpr int kBoxHalves = (kSweepThreads / 32) * kBoxNodes / kBoxP;
+static_assert(kBoxHalves * kBoxP == (kSweepThreads / 32) * kBoxNodes, "points and halves");
 constexpr double kBoxFar = 3.0;  // far: at least this many h from mid
 
 // A box's scratch lies in the node's slices of the next level's arrays,
@@ -77,9 +81,9 @@ enum BoxSum { kBoxSecular, kBoxLowner, kBoxRows };
 
 struct BoxSmem {
     double cosv[4 * kBoxP];               // cos(pi i / 48)
-    double val[4][kBoxP];                 // sums at the points
+    double val[kBoxHalves][4][kBoxP];     // sums at the points
     double coef[kSweepThreads / 32][4 * kBoxP]; // a warp's box
-    BoxHdr hdr;
+    double red[32];
 };
 
 // Poles of node list d[0, K) with d - mid < v (or <= v), by all threads.
@@ -110,7 +114,11 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
     const Ws &w = a.w;
     const LevelCtl *ctl = &w.hdr->lvl[a.k];
     const int boxes = ctl->items_c, b = ctl->box;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = threadIdx.x >> 5;
+    const int node0 = (warp / kBoxHalves) * kBoxNodes, half = warp % kBoxHalves;
+    // the warp's lanes among those that stride over the poles
+    const int lane = half * 32 + (threadIdx.x & 31);
+    constexpr int kStep = 32 * kBoxHalves;
     constexpr int NF = WHAT == kBoxSecular ? 4 : WHAT == kBoxLowner ? 1 : 3;
     for (int item = blockIdx.x; item < boxes; item += gridDim.x) {
         const int g = w.items_c[item];
@@ -147,19 +155,19 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
         if (!H.far(K)) {
             continue;
         }
-        double x[kBoxNodes], f[4][kBoxNodes];
+        double x[kBoxNodes], f[NF][kBoxNodes];
 #pragma unroll
         for (int u = 0; u < kBoxNodes; ++u) {
-            x[u] = H.h * S.cosv[2 * (warp * kBoxNodes + u) + 1];
+            x[u] = H.h * S.cosv[2 * (node0 + u) + 1];
 #pragma unroll
-            for (int i = 0; i < 4; ++i) {
+            for (int i = 0; i < NF; ++i) {
                 f[i][u] = WHAT == kBoxLowner ? 1.0 : 0.0;
             }
         }
-        if (WHAT == kBoxSecular) {
+        if constexpr (WHAT == kBoxSecular) {
             const double *pz = w.pz + po;
-#pragma unroll 2
-            for (int j = lane; j < H.nlo; j += 32) {
+#pragma unroll 4
+            for (int j = lane; j < H.nlo; j += kStep) {
                 const double d = __ldg(pd + j) - H.mid, z = __ldg(pz + j);
 #pragma unroll
                 for (int u = 0; u < kBoxNodes; ++u) {
@@ -168,8 +176,8 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
                     f[1][u] = fma(t, t, f[1][u]);
                 }
             }
-#pragma unroll 2
-            for (int j = H.nhi + lane; j < K; j += 32) {
+#pragma unroll 4
+            for (int j = H.nhi + lane; j < K; j += kStep) {
                 const double d = __ldg(pd + j) - H.mid, z = __ldg(pz + j);
 #pragma unroll
                 for (int u = 0; u < kBoxNodes; ++u) {
@@ -178,7 +186,7 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
                     f[3][u] = fma(t, t, f[3][u]);
                 }
             }
-        } else if (WHAT == kBoxLowner) {
+        } else if constexpr (WHAT == kBoxLowner) {
             const double *rdo = w.rdo + po, *rtau = w.rtau + po;
             // far poles by number: [0, low) and then [nhi, K)
             const int nl = H.low(), nf = nl + (K - H.nhi);
@@ -188,10 +196,10 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
                 *d = H.mid - __ldg(pd + j);
             };
             int i = lane;
-            for (; i + 32 < nf; i += 64) {
+            for (; i + kStep < nf; i += 2 * kStep) {
                 double n1, d1, n2, d2;
                 at(i, &n1, &d1);
-                at(i + 32, &n2, &d2);
+                at(i + kStep, &n2, &d2);
 #pragma unroll
                 for (int u = 0; u < kBoxNodes; ++u) {
                     f[0][u] *= lowner_pair(n1 + x[u], d1 + x[u], n2 + x[u], d2 + x[u]);
@@ -208,8 +216,8 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
         } else {
             const double *pw = w.pw + po, *pf = w.pf + po, *pl = w.pl + po;
             const int nf = H.nlo + (K - H.nhi);
-#pragma unroll 2
-            for (int i = lane; i < nf; i += 32) {
+#pragma unroll 4
+            for (int i = lane; i < nf; i += kStep) {
                 const int j = i < H.nlo ? i : H.nhi + (i - H.nlo);
                 const double d = __ldg(pd + j) - H.mid, wj = __ldcg(pw + j);
                 const double fj = __ldg(pf + j), lj = __ldg(pl + j);
@@ -228,8 +236,8 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
             for (int u = 0; u < kBoxNodes; ++u) {
                 const double v = WHAT == kBoxLowner ? group_prod(f[i][u], 32)
                                                     : group_sum(f[i][u], 32);
-                if (lane == 0) {
-                    S.val[i][warp * kBoxNodes + u] = v;
+                if ((threadIdx.x & 31) == 0) {
+                    S.val[half][i][node0 + u] = v;
                 }
             }
         }
@@ -240,7 +248,12 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
             double c = 0.0;
 #pragma unroll 4
             for (int k = 0; k < kBoxP; ++k) {
-                c = fma(S.val[i][k], S.cosv[(m * (2 * k + 1)) % (4 * kBoxP)], c);
+                double v = S.val[0][i][k];
+#pragma unroll
+                for (int h = 1; h < kBoxHalves; ++h) {
+                    v = WHAT == kBoxLowner ? v * S.val[h][i][k] : v + S.val[h][i][k];
+                }
+                c = fma(v, S.cosv[(m * (2 * k + 1)) % (4 * kBoxP)], c);
             }
             c *= (m == 0 ? 1.0 : 2.0) / kBoxP;
             double *to = WHAT == kBoxSecular ? (i < 2 ? w.nd : w.nf) + sb + kBoxP * (i & 1)
@@ -260,9 +273,9 @@ __device__ inline void box_runs(const KArgs &a, bool inner_only, Body body) {
     const LevelCtl *ctl = &w.hdr->lvl[a.k];
     const int tpr = ctl->tpr_w, items = ctl->items_w, b = ctl->box, Rw = 32 / tpr;
     const int warp = threadIdx.x >> 5;
-    // last runs first: the warp that has a merge's last root takes longest
     for (int it = (int)blockIdx.x * kWarpsPerBlock + warp; it < items;
          it += (int)gridDim.x * kWarpsPerBlock) {
+        // from the end: the blocks with the merges' last roots come last
         const int item = items - 1 - it;
         const int g = w.items_w[item];
         const NodeGeom G = node_geom(a.F, a.k, g);
@@ -281,6 +294,61 @@ __device__ inline void box_coef(double *dst, const double *src) {
     if (lane < kBoxP) {
         dst[lane] = __ldcg(src + lane);
     }
+}
+
+// body(G, g, K) for every merge of the level, one block each (the merges are
+// found by their first boxes).
+template <class Body>
+__device__ inline void box_merges(const KArgs &a, bool inner_only, Body body) {
+    const Ws &w = a.w;
+    const int boxes = w.hdr->lvl[a.k].items_c;
+    for (int item = blockIdx.x; item < boxes; item += gridDim.x) {
+        const int g = w.items_c[item];
+        if (item != w.pref_c[g]) {
+            continue;
+        }
+        const NodeGeom G = node_geom(a.F, a.k, g);
+        if (!(inner_only && G.depth == 0)) {
+            body(G, g, w.nK[g]);
+        }
+    }
+}
+
+// The last roots, each over all poles of its merge by a whole block (one
+// warp took 28 us for 8192 poles, longer than all other roots of the level).
+__device__ void box_last_root(const KArgs &a, BoxSmem &S) {
+    const Ws &w = a.w;
+    const double eps = DBL_EPSILON;
+    const int max_iter = w.hdr->max_iter;
+    box_merges(a, false, [&](const NodeGeom &G, int g, int K) {
+        const long long po = G.poff;
+        const double *pd = w.pd + po, *pz = w.pz + po;
+        SecRoot st;
+        sec_init(st, K - 1, K, pd, pz, w.nrho[g], w.nzn[g]);
+        while (st.stage != 2) {
+            SecSums sum;
+            sec_zero(sum);
+            secular_span(sum, st, 0, K, threadIdx.x, kSweepThreads, K - 2, K,
+                         [&](int j, double *d, double *z) {
+                             *d = __ldg(pd + j);
+                             *z = __ldg(pz + j);
+                         });
+            SecTot tot = sec_total(sum);
+            // every thread ends with the same totals, and so the same state
+            tot.sum = block_sum<kSweepThreads>(tot.sum, S.red);
+            tot.mag = block_sum<kSweepThreads>(tot.mag, S.red);
+            tot.dpsi = block_sum<kSweepThreads>(tot.dpsi, S.red);
+            tot.dphi = block_sum<kSweepThreads>(tot.dphi, S.red);
+            sec_bound(tot, K / kSweepThreads);
+            sec_after_sweep(st, tot, eps, max_iter);
+        }
+        if (threadIdx.x < 32) {
+            if (threadIdx.x == 0) {
+                secular_store(w, a, po, K - 1, st);
+            }
+            secular_diag_warp(w, a.k, threadIdx.x == 0, st);
+        }
+    });
 }
 
 __device__ void box_secular(const KArgs &a, BoxSmem &S) {
@@ -346,22 +414,6 @@ __device__ void box_secular(const KArgs &a, BoxSmem &S) {
             secular_store(w, a, po, r, st);
         }
         secular_diag_warp(w, a.k, active && l == 0, st);
-        if (r1 == K) {
-            // the last root, over all poles, by the whole warp
-            sec_init(st, K - 1, K, pd, pz, rho, zn);
-            while (st.stage != 2) {
-                SecSums sum;
-                sec_zero(sum);
-                secular_span(sum, st, 0, K, lane, 32, K - 2, K, ld);
-                SecTot tot = sec_total(sum);
-                sums_reduce(tot, 32);
-                sec_after_sweep(st, tot, eps, max_iter);
-            }
-            if (lane == 0) {
-                secular_store(w, a, po, K - 1, st);
-            }
-            secular_diag_warp(w, a.k, lane == 0, st);
-        }
     });
 }
 
@@ -384,7 +436,7 @@ __device__ void box_lowner(const KArgs &a, BoxSmem &S) {
         if (active) {
             const double di = __ldg(pd + i);
             int j = H.low() + l;
-#pragma unroll 2
+#pragma unroll 4
             for (; j + tpr < H.nhi; j += 2 * tpr) {
                 const int j2 = j + tpr;
                 const double dl = (di - __ldcg(rdo + j)) - __ldcg(rtau + j);
@@ -407,14 +459,58 @@ __device__ void box_lowner(const KArgs &a, BoxSmem &S) {
     });
 }
 
+// sum u^2, sum f u, sum l u of the root at (dorg, tau) over poles i, i + n,
+// ... below hi.
+__device__ __forceinline__ void rows_span(const Ws &w, long long po, double dorg, double tau,
+                                          int i, int hi, int n, double (&f)[3]) {
+    const double *pd = w.pd + po, *pw = w.pw + po, *pf = w.pf + po, *pl = w.pl + po;
+    auto add = [&](int j, double u) {
+        f[0] += u * u;
+        f[1] += __ldg(pf + j) * u;
+        f[2] += __ldg(pl + j) * u;
+    };
+#pragma unroll 4
+    for (; i + n < hi; i += 2 * n) {
+        double u, u2;
+        row_pair(__ldcg(pw + i), (__ldg(pd + i) - dorg) - tau, __ldcg(pw + i + n),
+                 (__ldg(pd + i + n) - dorg) - tau, &u, &u2);
+        add(i, u);
+        add(i + n, u2);
+    }
+    if (i < hi) {
+        const double dl = (__ldg(pd + i) - dorg) - tau;
+        add(i, dl != 0.0 ? __ldcg(pw + i) * brdc_rcp(dl) : 0.0);
+    }
+}
+
+__device__ __forceinline__ void rows_store(const Ws &w, long long po, int s,
+                                           const double (&f)[3]) {
+    const double nrm = sqrt(f[0]);
+    w.rf[po + s] = nrm > 0.0 ? f[1] / nrm : 0.0;
+    w.rl[po + s] = nrm > 0.0 ? f[2] / nrm : 0.0;
+}
+
 __device__ void box_rows(const KArgs &a, BoxSmem &S) {
     const Ws &w = a.w;
     const int lane = threadIdx.x & 31;
     double *cf = S.coef[threadIdx.x >> 5];
+    // the last roots by whole blocks
+    box_merges(a, true, [&](const NodeGeom &G, int g, int K) {
+        const long long po = G.poff;
+        double f[3] = {0.0, 0.0, 0.0};
+        rows_span(w, po, __ldcg(w.rdo + po + K - 1), __ldcg(w.rtau + po + K - 1), threadIdx.x, K,
+                  kSweepThreads, f);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+            f[c] = block_sum<kSweepThreads>(f[c], S.red);
+        }
+        if (threadIdx.x == 0) {
+            rows_store(w, po, K - 1, f);
+        }
+    });
     box_runs(a, true, [&](const NodeGeom &G, int g, int K, int r0, int Rw, int tpr, long long sb,
                           const BoxHdr &H) {
         const long long po = G.poff;
-        const double *pd = w.pd + po, *pw = w.pw + po, *pf = w.pf + po, *pl = w.pl + po;
         const bool far = H.far(K);
         if (far) {
             __syncwarp();
@@ -423,54 +519,29 @@ __device__ void box_rows(const KArgs &a, BoxSmem &S) {
             box_coef(cf + 2 * kBoxP, w.nf + sb);
             __syncwarp();
         }
-        // sums of root s over poles [lo, hi) by lanes l of n; far: the rest
-        auto rows = [&](int s, int l, int n, int lo, int hi, bool rest) {
-            double f[3] = {0.0, 0.0, 0.0};
-            if (s >= 0) {
-                const double dorg = __ldcg(w.rdo + po + s), tau = __ldcg(w.rtau + po + s);
-                auto add = [&](int i, double u) {
-                    f[0] += u * u;
-                    f[1] += __ldg(pf + i) * u;
-                    f[2] += __ldg(pl + i) * u;
-                };
-                int i = lo + l;
-#pragma unroll 2
-                for (; i + n < hi; i += 2 * n) {
-                    double u, u2;
-                    row_pair(__ldcg(pw + i), (__ldg(pd + i) - dorg) - tau, __ldcg(pw + i + n),
-                             (__ldg(pd + i + n) - dorg) - tau, &u, &u2);
-                    add(i, u);
-                    add(i + n, u2);
-                }
-                if (i < hi) {
-                    const double dl = (__ldg(pd + i) - dorg) - tau;
-                    add(i, dl != 0.0 ? __ldcg(pw + i) * brdc_rcp(dl) : 0.0);
-                }
-                if (rest) {
-                    const double t = ((dorg - H.mid) + tau) * H.ih;
-                    for (int q = l; q < 3; q += n) {
-                        const double v = box_eval(cf + q * kBoxP, t);
+        const int s = r0 + lane / tpr, l = lane & (tpr - 1);
+        const bool active = s < K - 1;
+        double f[3] = {0.0, 0.0, 0.0};
+        if (active) {
+            const double dorg = __ldcg(w.rdo + po + s), tau = __ldcg(w.rtau + po + s);
+            rows_span(w, po, dorg, tau, H.nlo + l, H.nhi, tpr, f);
+            if (far) {
+                const double t = ((dorg - H.mid) + tau) * H.ih;
+                for (int q = l; q < 3; q += tpr) {
+                    const double v = box_eval(cf + q * kBoxP, t);
 #pragma unroll
-                        for (int c = 0; c < 3; ++c) {
-                            f[c] += c == q ? v : 0.0;
-                        }
+                    for (int c = 0; c < 3; ++c) {
+                        f[c] += c == q ? v : 0.0;
                     }
                 }
             }
+        }
 #pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                f[c] = group_sum(f[c], n);
-            }
-            if (s >= 0 && l == 0) {
-                const double nrm = sqrt(f[0]);
-                w.rf[po + s] = nrm > 0.0 ? f[1] / nrm : 0.0;
-                w.rl[po + s] = nrm > 0.0 ? f[2] / nrm : 0.0;
-            }
-        };
-        const int s = r0 + lane / tpr;
-        rows(s < K - 1 ? s : -1, lane & (tpr - 1), tpr, H.nlo, H.nhi, far);
-        if (r0 + Rw >= K) {
-            rows(K - 1, lane, 32, 0, K, false);
+        for (int c = 0; c < 3; ++c) {
+            f[c] = group_sum(f[c], tpr);
+        }
+        if (active && l == 0) {
+            rows_store(w, po, s, f);
         }
     });
 }
@@ -497,6 +568,7 @@ __global__ void __launch_bounds__(kSweepThreads, 2) k_box(KArgs a, int rows, lon
     if (!grid_barrier(h, ctl)) {
         return;
     }
+    box_last_root(a, S);
     box_secular(a, S);
     if (!grid_barrier(h, ctl)) {
         return;
