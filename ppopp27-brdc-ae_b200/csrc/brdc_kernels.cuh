@@ -1515,6 +1515,30 @@ __device__ inline SecTot secular_shared(const SecRoot &st, const double *pd, con
     return sec_total(sum);
 }
 
+// The first sweep of a root, at the midpoint of its bracket: the update there
+// reads the sum and the sum of squares alone, so neither the sides nor the
+// moduli are kept (8 FP64 instructions a pole, not 10 or 11).
+__device__ inline SecTot secular_middle(const SecRoot &st, const double *pd, const double *pz,
+                                        int K, int l, int tpr, bool live) {
+    SecTot sum{};
+    if (live) {
+#pragma unroll 4
+        for (int j = l; j < K; j += tpr) {
+            const bool skip = (unsigned)(j - st.p) < 2u;
+            const double z = pz[j];
+            const double delta = sec_high((pd[j] - st.eorg_d) - st.etau, skip, 0x3ff00000);
+            const double t = sec_high(z * brdc_rcp(delta), skip, 0);
+            sum.sum = fma(z, t, sum.sum);
+            sum.dpsi = fma(t, t, sum.dpsi);
+        }
+    }
+    for (int o = tpr >> 1; o > 0; o >>= 1) {
+        sum.sum += __shfl_xor_sync(0xffffffffu, sum.sum, o);
+        sum.dpsi += __shfl_xor_sync(0xffffffffu, sum.dpsi, o);
+    }
+    return sum;
+}
+
 // A root's sums over its lanes with the bound of sec_bound (K poles).
 __device__ inline void sums_reduce_shared(SecTot &sum, int tpr, int K) {
     for (int o = tpr >> 1; o > 0; o >>= 1) {

@@ -547,12 +547,17 @@ __global__ void __launch_bounds__(kSubRows, 512 / kSubRows) k_subtree(SubArgs A)
             }
             // hardly a root converges before its third sweep: the first round
             // takes three, with no barrier, parking or list between them
-            for (int sweeps = round == 0 ? kSubFirstSweeps : 1; sweeps > 0; --sweeps) {
+            for (int left = round == 0 ? kSubFirstSweeps : 1; left > 0; --left) {
                 SecTot sum{};
-                if (st.stage != 2) {
-                    sum = secular_shared(st, pd, pz, Kr, l2, tp, rr < Kr - 2 ? rr : Kr - 2, rr + 1);
+                if (round == 0 && left == kSubFirstSweeps) {
+                    sum = secular_middle(st, pd, pz, Kr, l2, tp, act);
+                } else {
+                    if (st.stage != 2) {
+                        sum = secular_shared(st, pd, pz, Kr, l2, tp, rr < Kr - 2 ? rr : Kr - 2,
+                                             rr + 1);
+                    }
+                    sums_reduce_shared(sum, tp, Kr);
                 }
-                sums_reduce_shared(sum, tp, Kr);
                 if (st.stage != 2) {
                     sec_after_sweep(st, sum, eps, max_iter);
                 }
