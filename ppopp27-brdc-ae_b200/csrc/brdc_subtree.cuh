@@ -39,15 +39,6 @@ struct SubArgs {
     int leaves_done;          // the leaves were solved by k_leaf_full: read them
 };
 
-// Roots per warp at most in the barrier-free tail of the subtree's secular
-// rounds (the rounds stop once the live roots fit this many per warp).
-// Measured on B200 (uniform 65,536): 1 -> 0.846 ms, 4 -> 0.856, 8 -> 0.865,
-// 16 -> 0.914: repacking the live roots every round beats iterating
-// several of them per warp, whose lanes idle once their root converges.
-#ifndef BRDC_SUB_TAIL_ROOTS
-#define BRDC_SUB_TAIL_ROOTS 1
-#endif
-constexpr int kSubTailRoots = BRDC_SUB_TAIL_ROOTS;
 // Sweeps of the first round.  Measured on B200 (uniform 65,536): 1 584 us,
 // 2 586, 3 579, 4 592.
 constexpr int kSubFirstSweeps = 3;
@@ -476,55 +467,12 @@ __global__ void __launch_bounds__(kSubRows, 512 / kSubRows) k_subtree(SubArgs A)
         int cur = 0, round = 0;
         __syncthreads();
         while (nact > 0) {
-            if (nact <= kSubWarps * kSubTailRoots) {
-                // The last roots (the slow tail of the iteration): R per
-                // warp (the smallest power of two that covers them, dealt
-                // round robin over the warps), 32 / R lanes each, iterated
-                // to convergence with no barrier, parking or list between
-                // sweeps.  A lane group's lanes hold the same state (the
-                // butterfly sums are bit-identical); the warp loops until
-                // its last root converges, and the iteration cap ends it.
-                int R = 1;
-                while (R < kSubTailRoots && R * kSubWarps < nact) {
-                    R <<= 1;
-                }
-                const int lanes = 32 / R;
-                const int sub = lane / lanes, l2 = lane & (lanes - 1);
-                const int slot = sub * kSubWarps + (x >> 5);
-                const bool act = slot < nact;
-                const int code = act ? S.aq[cur][slot] : 0;
-                const int id = code & 0xffff, q = code >> 16;
-                const int rr = id - S.kpre[q], Kr = S.nK[q], sr = S.nstart[q];
-                const double *pd = S.pd + sr, *pz = S.pz + sr;
-                SecRoot st;
-                if (act) {
-                    sec_init(st, rr, Kr, pd, pz, S.nrho[q], S.nrinv[q], S.nzn[q]);
-                    if (round > 0) {
-                        sec_unpark(st, S.dyn[id]);
-                    }
-                } else {
-                    st.stage = 2;
-                }
-                for (;;) {
-                    SecTot sum{};
-                    const bool live = act && st.stage != 2;
-                    if (live) {
-                        sum = secular_shared(st, pd, pz, Kr, l2, lanes, rr < Kr - 2 ? rr : Kr - 2, rr + 1);
-                    }
-                    sums_reduce_shared(sum, lanes, Kr);
-                    if (live) {
-                        sec_after_sweep(st, sum, eps, max_iter);
-                    }
-                    if (__all_sync(0xffffffffu, !act || st.stage == 2)) {
-                        break;
-                    }
-                }
-                if (act && l2 == 0) {
-                    sec_park(st, S.dyn[id]);
-                }
-                __syncthreads();
-                break;
-            }
+            // The last roots (the slow tail of the iteration), one a warp:
+            // iterated to convergence with no barrier, parking or list
+            // between sweeps.  A lane group's lanes hold the same state (the
+            // butterfly sums are bit-identical), and the iteration cap ends
+            // the loop.
+            const bool tail = nact <= kSubWarps;
             int lg = 0;
             while (lg < 5 && nact << (lg + 1) <= kSubRows) {
                 ++lg;
@@ -547,9 +495,10 @@ __global__ void __launch_bounds__(kSubRows, 512 / kSubRows) k_subtree(SubArgs A)
             }
             // hardly a root converges before its third sweep: the first round
             // takes three, with no barrier, parking or list between them
-            for (int left = round == 0 ? kSubFirstSweeps : 1; left > 0; --left) {
+            const int first = round == 0 ? kSubFirstSweeps : 1;
+            for (int left = first; left > 0 || tail; --left) {
                 SecTot sum{};
-                if (round == 0 && left == kSubFirstSweeps) {
+                if (round == 0 && left == first) {
                     sum = secular_middle(st, pd, pz, Kr, l2, tp, act);
                 } else {
                     if (st.stage != 2) {
@@ -561,6 +510,9 @@ __global__ void __launch_bounds__(kSubRows, 512 / kSubRows) k_subtree(SubArgs A)
                 if (st.stage != 2) {
                     sec_after_sweep(st, sum, eps, max_iter);
                 }
+                if (tail && __all_sync(kFull, st.stage == 2)) {
+                    break;
+                }
             }
             // one barrier per round: round r appends to qc[r % 3], and
             // qc[(r+2) % 3], last read in round r-1, is cleared after this
@@ -569,6 +521,10 @@ __global__ void __launch_bounds__(kSubRows, 512 / kSubRows) k_subtree(SubArgs A)
             const bool lead = act && l2 == 0;
             if (lead) {
                 sec_park(st, S.dyn[id]);
+            }
+            if (tail) {
+                __syncthreads();
+                break;
             }
             const bool more = lead && st.stage != 2;
             const unsigned mb = __ballot_sync(0xffffffffu, more);
