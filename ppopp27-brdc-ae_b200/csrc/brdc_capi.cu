@@ -504,15 +504,19 @@ void mark(brdc_handle h, int slot) {
 }
 
 // Subtree depth of a solve: the handle's setting, or by default the depth
-// measured fastest on B200: 5 for a batch with at least two 512-row
-// subtrees per SM (the subtrees fill the GPU), otherwise by the forest's
-// tallest instance (3 up to 11 levels, i.e. n <= 32768; 5 above).
+// measured fastest on B200.  Batches (us a solve at depths 3, 4, 5): 64
+// instances up to 300 rows (7,000 rows) 153, 165, 181; up to 4000 rows
+// (47,000) 412, 332, 355; 1000 up to 500 rows (168,000) 787, 606, 792; so 4
+// once their 256-row subtrees come near half the SMs.  Large batches of long
+// instances, of all families mixed (5.8 million rows, 1400 a matrix) 48,052,
+// 36,601, 35,399: 5.  A single matrix goes by its height: 3 up to 11 levels
+// (n <= 32768), 5 above.
 int effective_sub_levels(brdc_handle h, const HostForest &hf) {
     if (h->sub_levels >= 0) {
         return h->sub_levels;
     }
-    if (hf.B > 1 && hf.total_n >= 512LL * 2 * h->sm_count) {
-        return 5;
+    if (hf.B > 1 && hf.total_n >= 112LL * h->sm_count) {
+        return hf.total_n >= 1024LL * std::max(h->sm_count, hf.B) ? 5 : 4;
     }
     // measured on B200 (uniform and normal, ms per solve): depth 3 is the
     // fastest up to n = 32,768 (11 levels; 32,768: 0.583 against 0.609 at

@@ -435,7 +435,7 @@ __host__ __device__ inline int sec_after_sweep(SecRoot &r, const SecTot &s,
         } else {
             const double del = r.dq - r.dp;
             const double mid = r.etau;
-            const double w = c + r.zp2 / ((r.dp - r.dq) - mid) + r.zq2 / (-mid);
+            const double w = c - r.zp2 * brdc_rcp(del + mid) - r.zq2 * brdc_rcp(mid);
             if (w <= 0.0) {
                 r.lo = mid;
                 r.hi = r.hi0;
@@ -448,8 +448,8 @@ __host__ __device__ inline int sec_after_sweep(SecRoot &r, const SecTot &s,
                 const double a = c * del - r.zp2 - r.zq2;
                 const double b = r.zq2 * del;
                 const double disc = sqrt(fabs(a * a + 4.0 * b * c));
-                const double t2 = (a <= 0.0) ? (disc - a) / (2.0 * c)
-                                             : 2.0 * b / (a + disc);
+                const double t2 = (a <= 0.0 ? disc - a : 2.0 * b) *
+                                  brdc_rcp(a <= 0.0 ? 2.0 * c : a + disc);
                 if (t2 > r.lo && t2 <= r.hi) {
                     tau = t2;
                 } else if (!(t2 > r.lo)) {
