@@ -212,7 +212,7 @@ def run_reference_arm(args, rank):
 def run_profile_case(spec):
     """One or more plain solves of a seeded instance with the library's
     default launch shapes, nothing else on the GPU: solve i launches k_init,
-    k_norm, k_subtree, then per level above the subtree k_level and k_sweeps
+    k_norm, k_subtree, then per level above the subtree k_level and k_box
     (from the second solve on as a replay of the library's graph of the
     same launches), so a kernel's launch index is known in advance."""
     import torch
@@ -1179,10 +1179,17 @@ def work_model(diag, fused):
     for k, lv in enumerate(levels):
         kk = max(lv["dd_after_sum"], 1)
         sweeps = lv["secular_iter_sum"] / kk + 1.0
-        sec = 8.0 * lv["dd_after_sq_sum"] * sweeps
+        far, near = 0.0, float(lv["dd_after_sq_sum"])
+        kmax = lv["dd_after_max"]
+        if kmax > 512 and lv["size_sum"] > 1024 * lv["merge_count"]:
+            # k_box: 24 points per box of b poles for the far sums, once, and
+            # the near poles, about 3 b
+            b = 64 if kmax <= 8192 else 128 if kmax <= 16384 else 256
+            far, near = 24.0 / b * near, min(near, 3.0 * b * kk)
+        sec = 8.0 * (far + near * sweeps)
         inner = k < nlev - 1
-        low = 4.0 * lv["dd_after_sq_sum"] if inner else 0.0
-        rows = 10.0 * lv["dd_after_sq_sum"] if inner else 0.0
+        low = 4.0 * (far + near) if inner else 0.0
+        rows = 10.0 * (far + near) if inner else 0.0
         per.append((sec, low, rows))
     sub = leaf + sum(a + b + c for a, b, c in per[:fused])
     return sub, per
@@ -1195,9 +1202,9 @@ def roofline(diag, phase, n, total_ms=None, fused=0, level_rows=0):
     level: d, z, two rows read and written, an index).  Candidates: the
     subtree kernel (leaves and the lowest levels), k_level (the levels whose
     largest merge has at most `level_rows` rows: its phase column holds the
-    whole level), k_sweeps (roots, Loewner, rows and placement of the other
-    levels, and of the merges k_level hands on), and the per-level merge and
-    deflation."""
+    whole level), k_box (the merges k_level hands on; with the fused levels
+    off k_sweeps, every merge's roots, Loewner weights, rows and placement),
+    and the per-level merge and deflation."""
     hbm, hbm_kind = measured_peaks()
     levels = diag["level"]
     fp64_peak = fp64_peak_gflops()
@@ -1229,7 +1236,7 @@ def roofline(diag, phase, n, total_ms=None, fused=0, level_rows=0):
     cand = {
         "k_subtree": (phase["leaf_ms"], sub_flops, "fp64"),
         "k_level": (lvl_ms[0], lvl_work[0], "fp64"),
-        "k_sweeps": (sw_ms, sw_work, "fp64"),
+        "k_box": (sw_ms, sw_work, "fp64"),
         "k_merge+k_merge_deflate": (lvl_ms[1], lvl_work[1], "hbm"),
     }
     name = max(cand, key=lambda k: cand[k][0])
@@ -1255,7 +1262,7 @@ def roofline(diag, phase, n, total_ms=None, fused=0, level_rows=0):
 # DRAM bytes (read + write) of one launch, from the ncu captures summarised
 # in profiles/ (uniform N=65536): the working set is L2-resident, so DRAM
 # sees little more than the first touch of the inputs.
-KERNEL_TRAFFIC = {"k_subtree": 1240320}
+KERNEL_TRAFFIC = {"k_subtree": 1185536, "k_level": 1734400}
 
 # the library's default launch shapes (brdc_tuning defaults)
 DEFAULT_TUNING = {"subtree_levels": -1, "deflate_cluster": 16, "sweep_lanes_target": 303104,

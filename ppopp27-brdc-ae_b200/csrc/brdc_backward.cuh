@@ -21,7 +21,7 @@
 // four sums over the roots (k_bw_poles), written pair by pair so that a
 // root lying within z_o^2 of its origin pole o costs no cancellation.  Deflation is undone by reversing
 // each Givens chain (k_bw_undeflate), the merge permutation by a gather;
-// the leaves by the eigenvector adjoint of their 16x16 Jacobi solve
+// the leaves by the eigenvector adjoint of their 16x16 eigenvectors
 // (k_bw_leaf).  d(L)/dE at a cut collects 2*sign(E)*dL/drho from its merge
 // and -sign(E)*dL/dD' from the two leaf corners the cut modified
 // (k_bw_cuts), in a fixed order, so the adjoint is bitwise reproducible.

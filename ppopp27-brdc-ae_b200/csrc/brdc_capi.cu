@@ -2,7 +2,7 @@
 //
 // The driver plans a forest (one or many tridiagonals), carves the caller's
 // workspace, and enqueues the leaves and lowest levels (k_subtree), then per
-// level either the fused k_level (with k_sweeps for merges that keep many
+// level either the fused k_level (with k_box for merges that keep many
 // poles) or k_merge, the deflation and k_sweeps.  All launch shapes depend
 // only on the orders, never on data, and no call synchronises the stream,
 // so a solve can be captured in a CUDA graph.  Data-dependent sizes (deflation counts K) travel from kernel to

@@ -89,7 +89,7 @@ struct LevelCtl {
     int items_c;     // CTA work items of the level
     int total_k;
     int nbig;        // merges k_level left to k_box (K > kLvlMaxK)
-    unsigned bar_count; // grid barrier of k_sweeps: arrivals, generation
+    unsigned bar_count; // grid barrier of k_sweeps and k_box: arrivals, generation
     unsigned bar_gen;
     int citem;       // next CTA-role item of the secular phase (taken by atomicAdd)
     int box;         // poles per box of the merges k_box takes
@@ -125,7 +125,7 @@ enum DeviceError : int {
 
 // A solve whose status word is set (non-finite input, a wait that ran out)
 // does no further work: every kernel after the one that set it returns at
-// once.  Only k_norm and k_sweeps set the word, and every later kernel
+// once.  Only k_norm, k_sweeps and k_box set the word, and every later kernel
 // waits for them to finish before it reads it, so all CTAs of a kernel read
 // the same value (no cluster or grid barrier can lose a member to it).
 #if defined(__CUDACC__)
