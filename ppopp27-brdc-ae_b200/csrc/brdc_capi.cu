@@ -2377,7 +2377,7 @@ namespace {
 // products (n x Kmax each), the GEMM pointer tables, the row signs and the
 // per-level Kmax.
 struct VecLayout {
-    size_t ckpt, qa, qb, mm, sgn, kmax, rows, cnt, total;
+    size_t ckpt, qa, qb, mm, sgn, rows, cnt, total;
 };
 
 VecLayout vec_layout(const HostForest &hf, long long n) {
@@ -2388,10 +2388,9 @@ VecLayout vec_layout(const HostForest &hf, long long n) {
     v.qb = align_up(half);
     v.mm = align_up((size_t)n * (size_t)n * sizeof(double));
     v.sgn = align_up(sizeof(double) * (size_t)n);
-    v.kmax = align_up(sizeof(int) * (size_t)(hf.max_levels + 1));
     v.rows = align_up(sizeof(int) * (size_t)n);
     v.cnt = align_up(sizeof(int) * 2 * (size_t)(hf.nn0 + 1));
-    v.total = v.ckpt + v.qa + v.qb + v.mm + v.sgn + v.kmax + v.rows + v.cnt;
+    v.total = v.ckpt + v.qa + v.qb + v.mm + v.sgn + v.rows + v.cnt;
     return v;
 }
 
@@ -2452,10 +2451,9 @@ extern "C" brdc_status brdc_dstebr_vectors(brdc_handle h, int64_t n, const doubl
     double *qb = reinterpret_cast<double *>(base + V.qa);
     double *M = reinterpret_cast<double *>(base + V.qa + V.qb);
     double *sgn = reinterpret_cast<double *>(base + V.qa + V.qb + V.mm);
-    int *dkmax = reinterpret_cast<int *>(base + V.qa + V.qb + V.mm + V.sgn);
-    int *vrows = reinterpret_cast<int *>(base + V.qa + V.qb + V.mm + V.sgn + V.kmax);
-    int *vcnt = reinterpret_cast<int *>(base + V.qa + V.qb + V.mm + V.sgn + V.kmax + V.rows);
-    k_vec_signs<<<1, 1024, 0, s>>>(d_E, n, sgn);
+    int *vrows = reinterpret_cast<int *>(base + V.qa + V.qb + V.mm + V.sgn);
+    int *vcnt = reinterpret_cast<int *>(base + V.qa + V.qb + V.mm + V.sgn + V.rows);
+    launch_pdl(k_vec_signs, 1, 1024, s, d_E, n, sgn);
     BRDC_CUDA(h, "brdc.vectors.signs", cudaGetLastError());
     const int Lv = hf.max_levels;
     long long eg = (n + 7) / 8; // one warp per slot, 8 warps a block
@@ -2464,7 +2462,7 @@ extern "C" brdc_status brdc_dstebr_vectors(brdc_handle h, int64_t n, const doubl
     zg = std::max<long long>(1, std::min<long long>(zg, (long long)h->sm_count * 16));
     if (Lv == 0) {
         // one leaf: its eigenvector matrix (ld 16) is the answer
-        k_vec_out<<<(unsigned)zg, 256, 0, s>>>(w.leafv, 16, n, sgn, d_Z, ldz);
+        launch_pdl(k_vec_out, zg, 256, s, w.leafv, 16LL, n, sgn, d_Z, ldz);
         BRDC_CUDA(h, "brdc.vectors.leaf", cudaGetLastError());
         return BRDC_STATUS_SUCCESS;
     }
@@ -2479,16 +2477,15 @@ extern "C" brdc_status brdc_dstebr_vectors(brdc_handle h, int64_t n, const doubl
             kmax[k] = hf.level_mmax[k];
         }
     } else {
-        BRDC_CUDA(h, "brdc.vectors.kmax_zero", cudaMemsetAsync(dkmax, 0, sizeof(int) * Lv, s));
-        for (int k = 0; k < Lv; ++k) {
-            Ws wl = w;
-            level_view(hf, L, w, k, &wl);
-            k_vec_kmax<<<1, 256, 0, s>>>(wl.nK, hf.level_nodes[k], dkmax + k);
-        }
-        BRDC_CUDA(h, "brdc.vectors.kmax", cudaGetLastError());
+        // the level counters of the values solve hold it
+        std::vector<brdc_level_diagnostics> dg(Lv);
         BRDC_CUDA(h, "brdc.vectors.kmax_read",
-                  cudaMemcpyAsync(kmax.data(), dkmax, sizeof(int) * Lv, cudaMemcpyDeviceToHost, s));
+                  cudaMemcpyAsync(dg.data(), w.hdr->diag, sizeof(dg[0]) * Lv,
+                                  cudaMemcpyDeviceToHost, s));
         BRDC_CUDA(h, "brdc.vectors.kmax_sync", cudaStreamSynchronize(s));
+        for (int k = 0; k < Lv; ++k) {
+            kmax[k] = dg[k].dd_after_max;
+        }
         // a failed values solve (its status word set) leaves the counts
         // unwritten: keep the products inside their buffers whatever was read
         for (int k = 0; k < Lv; ++k) {
@@ -2521,15 +2518,16 @@ extern "C" brdc_status brdc_dstebr_vectors(brdc_handle h, int64_t n, const doubl
         va.rows = vrows;
         va.cnt = vcnt;
         if (top) {
-            k_vec_lowner<<<(unsigned)std::max<long long>(1, std::min<long long>((n + 7) / 8, h->sm_count * 8)),
-                           256, 0, s>>>(va);
+            launch_pdl(k_vec_lowner,
+                       std::max<long long>(1, std::min<long long>((n + 7) / 8, h->sm_count * 8)),
+                       256, s, va);
             BRDC_CUDA(h, "brdc.vectors.lowner", cudaGetLastError());
         }
         // M needs no clearing: k_vec_build writes every row of a root
         // column that k_vec_gemm reads (the poles and the members rotated
         // into them, its listed rows), and nothing else of M is read
         // root columns of M; the deflated eigenvectors straight to the blocks
-        k_vec_build<<<(unsigned)eg, 256, 0, s>>>(va, n);
+        launch_pdl(k_vec_build, eg, 256, s, va, n);
         BRDC_CUDA(h, "brdc.vectors.build", cudaGetLastError());
         if (Km == 0) {
             qprev = qcur;
@@ -2540,14 +2538,17 @@ extern "C" brdc_status brdc_dstebr_vectors(brdc_handle h, int64_t n, const doubl
         // the roots: blockdiag(Q_left, Q_right) * M[:, :K] per node over the
         // surviving rows of M, each column written to its place (k_vec_gemm,
         // FP64 tensor cores)
-        k_vec_rows<256><<<(unsigned)hf.level_nodes[k], 256, 0, s>>>(va);
+        launch_pdl(k_vec_rows<256>, hf.level_nodes[k], 256, s, va);
         BRDC_CUDA(h, "brdc.vectors.rows", cudaGetLastError());
         {
             const long long half_rows = (mmax + 1) / 2;
             const dim3 grid((unsigned)((half_rows + kVgBM - 1) / kVgBM),
                             (unsigned)((Km + kVgBN - 1) / kVgBN),
                             (unsigned)(2 * hf.level_nodes[k]));
-            k_vec_gemm<<<grid, kVgThreads, 0, s>>>(va);
+            cudaLaunchAttribute at[1];
+            cudaLaunchConfig_t cfg = plain_config(1, kVgThreads, 0, s, at);
+            cfg.gridDim = grid;
+            cudaLaunchKernelEx(&cfg, k_vec_gemm, va);
             BRDC_CUDA(h, "brdc.vectors.gemm", cudaGetLastError());
         }
         qprev = qcur;

@@ -59,6 +59,7 @@ struct VArgs {
 // Loewner weights of the instance-root merges, which the values solve
 // skips (no parent reads their rows): one warp per pole.
 __global__ void __launch_bounds__(256) k_vec_lowner(VArgs a) {
+    pdl_begin();
     if (halted(a.w.hdr)) {
         return;
     }
@@ -125,6 +126,7 @@ __device__ inline int vec_pos(const Ws &w, long long gs, long long po, int s, in
 // eigenvector (small-z) or a short rotation combination of some (rotated
 // out), written straight to its place in the node's block.  M must be zero.
 __global__ void __launch_bounds__(256) k_vec_build(VArgs a, long long total_n) {
+    pdl_begin();
     if (halted(a.w.hdr)) {
         return;
     }
@@ -262,6 +264,7 @@ __global__ void __launch_bounds__(256) k_vec_build(VArgs a, long long total_n) {
 // uses the deflation (it multiplies only the non-deflated columns of Q).
 template <int T>
 __global__ void __launch_bounds__(T) k_vec_rows(VArgs a) {
+    pdl_begin();
     if (halted(a.w.hdr)) {
         return;
     }
@@ -342,6 +345,7 @@ __device__ __forceinline__ void dmma884(double (&c)[2], double a, double b) {
 }
 
 __global__ void __launch_bounds__(kVgThreads) k_vec_gemm(VArgs a) {
+    pdl_begin();
     if (halted(a.w.hdr)) {
         return;
     }
@@ -461,26 +465,13 @@ __global__ void __launch_bounds__(kVgThreads) k_vec_gemm(VArgs a) {
     }
 }
 
-// Largest K over one level's merges, for the host to size the products.
-__global__ void __launch_bounds__(256) k_vec_kmax(const int *nK, int nodes, int *kmax) {
-    int mx = 0;
-    for (int g = threadIdx.x; g < nodes; g += blockDim.x) {
-        mx = max(mx, nK[g]);
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        atomicMax(kmax, mx);
-    }
-}
-
 // The top node's eigenvectors into Z (ld ldz) with the signs of E: the
 // solve works on |E|, and T = S |T| S with S = diag(s), s_0 = 1,
 // s_{i+1} = s_i sign(E_i) (+1 for E_i = 0), i.e. s_i = (-1)^(negative E_j,
 // j < i).  One block: each thread counts the negatives of a contiguous
 // chunk, a block scan gives every chunk its parity.
 __global__ void __launch_bounds__(1024) k_vec_signs(const double *E, long long n, double *sgn) {
+    pdl_begin();
     __shared__ int iscan[32];
     const long long chunk = (n + 1023) / 1024;
     const long long lo = (long long)threadIdx.x * chunk;
@@ -499,6 +490,7 @@ __global__ void __launch_bounds__(1024) k_vec_signs(const double *E, long long n
 
 __global__ void __launch_bounds__(256) k_vec_out(const double *Q, long long ldq, long long n,
                                                  const double *sgn, double *Z, long long ldz) {
+    pdl_begin();
     const long long total = n * n;
     for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
