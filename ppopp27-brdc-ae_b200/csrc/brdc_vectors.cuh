@@ -118,6 +118,8 @@ __device__ inline int vec_pos(const Ws &w, long long gs, long long po, int s, in
     return q + upper_bound_d(rl, K, gdl[q]) + upper_bound_d(zdl, ndz, gdl[q]);
 }
 
+constexpr int kVecBatch = 8; // rows a lane of k_vec_build copies at once
+
 // One warp per slot of the level (lanes over rows and poles).  A root s
 // writes its column of M at column s (u_i = w_i / delta_i(s) over the
 // poles, normalised, then the chains undone on the rows -- chains touch
@@ -205,13 +207,31 @@ __global__ void __launch_bounds__(256) k_vec_build(VArgs a, long long total_n) {
                             : (left ? a.child + gs * a.child_stride + (long long)e * m1
                                     : a.child + (gs + m1) * a.child_stride +
                                           (long long)(e - m1) * (m - m1));
-            for (int r = lane; r < m; r += 32) {
-                double v = 0.0;
-                if (r >= r0 && r < r1) {
-                    v = c[r - r0];
-                    v = a.top ? v * a.sgn[r] : v;
+            // Eight loads are issued before their stores: one at a time, each
+            // row of the warp waited for the last (n = 8192, all levels: 485 -> 431 us).
+            for (int r = lane; r < r0; r += 32) {
+                dst[r] = 0.0;
+            }
+            for (int r = r1 + lane; r < m; r += 32) {
+                dst[r] = 0.0;
+            }
+            for (int b = r0 + lane; b < r1; b += 32 * kVecBatch) {
+                double v[kVecBatch];
+#pragma unroll
+                for (int q = 0; q < kVecBatch; ++q) {
+                    const int r = b + 32 * q;
+                    v[q] = r < r1 ? __ldg(c + (r - r0)) : 0.0;
+                    if (a.top && r < r1) {
+                        v[q] *= __ldg(a.sgn + r);
+                    }
                 }
-                dst[r] = v;
+#pragma unroll
+                for (int q = 0; q < kVecBatch; ++q) {
+                    const int r = b + 32 * q;
+                    if (r < r1) {
+                        dst[r] = v[q];
+                    }
+                }
             }
             continue;
         }
