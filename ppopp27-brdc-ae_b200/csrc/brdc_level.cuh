@@ -437,10 +437,15 @@ __device__ void level_load_active(LvlSmem &S, const Ws &w, long long gs, int Kz,
 // Close-pole chains and the poles of an active list of Kz <= kLvlMaxK entries
 // in this CTA's pd .. gmark: every CTA of the cluster does them for itself,
 // CTA 0 (`writer`) writes the lists.  pd, pz, pf and pl end as the K poles;
-// returns sum z^2 over them.
+// returns sum z^2 over them.  `loaded`: the entries came from the active list
+// in global memory (level_load_active), which holds them already; only
+// rotations change it, and CTA 0 writes those back after a cluster barrier,
+// when every CTA has its copy of the list.  All CTAs walk the same list, so
+// all of them find rotations (and take the barrier) or none does.
 template <int T>
-__device__ double level_poles(LvlSmem &S, const Ws &w, long long gs, long long po, int Kz,
-                              double tol, bool writer, bool keep, int big_k, int *K_out) {
+__device__ double level_poles(LvlSmem &S, cooperative_groups::cluster_group &cl, const Ws &w,
+                              long long gs, long long po, int Kz, double tol, bool writer,
+                              bool loaded, bool keep, int big_k, int *K_out) {
     const int x = threadIdx.x;
     // the walk on the shared lists; the rotations' own record is CTA 0's
     Ws v = w;
@@ -454,10 +459,13 @@ __device__ double level_poles(LvlSmem &S, const Ws &w, long long gs, long long p
     v.gs = writer ? w.gs + gs : S.stage + kLvlMaxK;
     v.gr = writer ? w.gr + gs : S.stage + 2 * kLvlMaxK;
     const bool rot = __syncthreads_or(defl_close_walk<T>(v, 0, Kz, tol, 0, Kz));
-    if (writer && keep) {
+    if (keep && loaded && rot) {
+        cl.sync();
+    }
+    if (writer && keep && (rot || !loaded)) {
+        // what the adjoint and the vectors read of the list (d and z are not
+        // among it)
         for (int i = x; i < Kz; i += T) {
-            w.ad[gs + i] = S.pd[i];
-            w.az[gs + i] = S.pz[i];
             w.af[gs + i] = S.pf[i];
             w.al[gs + i] = S.pl[i];
             w.amap[gs + i] = S.amap[i];
@@ -797,7 +805,8 @@ __global__ void __launch_bounds__(T, 1) k_level(KArgs a) {
     double tol;
     int K = 0, Kz = 0;
     double zn = 0.0;
-    bool local = false; // this CTA's shared memory holds the poles
+    bool local = false;  // this CTA's shared memory holds the poles
+    bool loaded = false; // from the active list in global memory
     if (m <= kLvlLocalRows) {
         Kz = level_merge_local<T>(S, buf, w, gs, m1, m, e0, e1, rho, maxd, keep, &tol);
         local = Kz <= kLvlMaxK;
@@ -857,7 +866,7 @@ __global__ void __launch_bounds__(T, 1) k_level(KArgs a) {
             // few poles: every CTA takes the list and goes on for itself,
             // with no more counts to exchange
             level_load_active<T>(S, w, gs, Kz, keep);
-            local = true;
+            local = loaded = true;
         } else if (solo) {
             if (rank == 0) {
                 defl_close_walk<T>(w, gs, Kz, tol, 0, Kz);
@@ -919,7 +928,7 @@ __global__ void __launch_bounds__(T, 1) k_level(KArgs a) {
         }
     }
     if (local) {
-        zn = level_poles<T>(S, w, gs, G.poff, Kz, tol, rank == 0, keep, a.big_k, &K);
+        zn = level_poles<T>(S, cl, w, gs, G.poff, Kz, tol, rank == 0, loaded, keep, a.big_k, &K);
     }
     if (rank == 0 && x == 0) {
         w.nK[g] = K;
