@@ -1157,11 +1157,13 @@ def work_model(diag, fused):
     """Algorithmic FP64 work of the solve from the solver's own counters
     (a divide or square root counts as one flop, an FMA as two):
       leaf Jacobi     (12 s + 15) flops per rotation, s(s-1)/2 rotations a
-                      sweep, summed over the leaves with the sweeps each
-                      leaf's half-warp ran; leaves solved one eigenpair per
-                      lane: per pair ten evaluations of det(T - x) of 8
-                      (s - 1) flops, 26 s for the vector and its residual,
-                      4 s^2 for the orthogonality correction
+                      sweep, summed over the sweeps the leaves took
+      leaf pairs      of the leaves that took no Jacobi, per eigenpair: ten
+                      evaluations of det(T - x) of 8 (s - 1) flops, 26 s for
+                      the vector and its residual, 4 s^2 for the
+                      orthogonality correction.  The counters hold the sum
+                      of the sweeps and the slowest leaf's, so the leaves
+                      that took Jacobi are counted as sum / max
       secular         8 flops per pole-root pair and sweep; sweeps per root
                       = its iterations + the initial midpoint sweep
       Loewner         4 flops per pair (inner merges only)
@@ -1172,9 +1174,9 @@ def work_model(diag, fused):
     leaves = diag["leaf_count"]
     s = 16
     sweeps = diag["leaf_sweeps_sum"]
+    jacobi = -(-sweeps // max(diag["leaf_sweeps_max"], 1))
     leaf = sweeps * (s * (s - 1) / 2) * (12 * s + 15)
-    if sweeps == 0:  # no leaf took Jacobi
-        leaf = leaves * s * (10 * 8 * (s - 1) + 26 * s + 4 * s * s)
+    leaf += (leaves - jacobi) * s * (10 * 8 * (s - 1) + 26 * s + 4 * s * s)
     per = []
     for k, lv in enumerate(levels):
         kk = max(lv["dd_after_sum"], 1)
