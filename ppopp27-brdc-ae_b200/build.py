@@ -55,10 +55,11 @@ def build(force: bool = False, verbose: bool = False) -> str:
             cmd.insert(1, "-Xptxas=-v")
         subprocess.run(cmd, check=True)
     cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
-    hdeps = [os.path.join(CSRC, f) for f in ("host_check.cpp", "brdc_secular.cuh", "brdc_leaf.cuh")]
+    hdeps = [os.path.join(CSRC, f) for f in ("host_check.cpp", "brdc_secular.cuh", "brdc_leaf.cuh",
+                                               "brdc_device_cache.h")]
     if force or _stale(HOSTLIB, hdeps):
         subprocess.run(
-            [cxx, "-O2", "-fPIC", "-shared", "-std=c++17", "-o", HOSTLIB,
+            [cxx, "-O2", "-fPIC", "-shared", "-std=c++17", "-pthread", "-o", HOSTLIB,
              os.path.join(CSRC, "host_check.cpp")],
             check=True,
         )

@@ -11,6 +11,8 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
+#include <atomic>
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -21,6 +23,7 @@
 #include "../../include/brdc_lapack.h"
 #include "brdc_backward.cuh"
 #include "brdc_box.cuh"
+#include "brdc_device_cache.h"
 #include "brdc_level.cuh"
 #include "brdc_vectors.cuh"
 #include "brdc_subtree.cuh"
@@ -393,28 +396,21 @@ cudaLaunchConfig_t cluster_config(unsigned grid, int C, cudaStream_t s, cudaLaun
 // Largest cluster (8, 4, 2) of 1024-thread deflation CTAs the device can
 // schedule; 1 when none.  Asked once per device.
 int max_defl_cluster(int device) {
-    static int cached[64];
-    static bool done[64];
-    if (device < 0 || device >= 64) {
-        return 1;
-    }
-    if (!done[device]) {
-        int best = 1;
+    static DeviceCache<int> cache;
+    const int best = cache.get(device, [](int) {
         for (int C = 8; C >= 2; C >>= 1) {
             cudaLaunchAttribute at[1];
             cudaLaunchConfig_t cfg = cluster_config((unsigned)C, C, nullptr, at);
             int n = 0;
             if (cudaOccupancyMaxActiveClusters(&n, k_merge_deflate_cl<1024>, &cfg) == cudaSuccess &&
                 n > 0) {
-                best = C;
-                break;
+                return C;
             }
             cudaGetLastError();
         }
-        cached[device] = best;
-        done[device] = true;
-    }
-    return cached[device];
+        return 1;
+    });
+    return std::max(best, 1);
 }
 
 // Returns the number of kernels launched.
@@ -463,7 +459,7 @@ int launch_merge_deflate(brdc_handle h, const KArgs &a0, int mmax, cudaStream_t 
 
 constexpr size_t smem_tiles(int na) { return sizeof(double) * 2 * na * kTile; }
 
-bool g_attr_done = false;
+std::atomic<bool> g_attr_done{false};
 
 cudaError_t set_attrs() {
     if (g_attr_done) {
@@ -527,54 +523,46 @@ int effective_sub_levels(brdc_handle h, const HostForest &hf) {
 // Clusters of C = 1, 2, 4, 8, 16 k_level CTAs the device holds at once
 // (0: C not schedulable).  Asked once per device (after set_attrs, which
 // sizes its shared memory and allows the non-portable size 16).
-const int *level_clusters(int device) {
-    static int cached[64][5];
-    static bool done[64];
-    static const int none[5] = {0, 0, 0, 0, 0};
-    if (device < 0 || device >= 64) {
-        return none;
-    }
-    if (!done[device]) {
+std::array<int, 5> level_clusters(int device) {
+    static DeviceCache<std::array<int, 5>> cache;
+    return cache.get(device, [](int) {
+        std::array<int, 5> act{};
         for (int q = 0; q < 5; ++q) {
             const int C = 1 << q;
             cudaLaunchAttribute at[1];
             cudaLaunchConfig_t cfg = cluster_config((unsigned)C, C, nullptr, at);
             cfg.blockDim = dim3(kLvlThreads);
             cfg.dynamicSmemBytes = sizeof(LvlSmem);
-            int n = 0;
-            if (cudaOccupancyMaxActiveClusters(&n, k_level<kLvlThreads>, &cfg) != cudaSuccess) {
+            if (cudaOccupancyMaxActiveClusters(&act[q], k_level<kLvlThreads>, &cfg) !=
+                cudaSuccess) {
                 cudaGetLastError();
-                n = 0;
+                act[q] = 0;
             }
-            cached[device][q] = n;
         }
-        done[device] = true;
-    }
-    return cached[device];
+        return act;
+    });
 }
 
-// Resident k_sweeps blocks per SM (without / with the CTA-role tiles), once
-// per device; 0 when the device has no cooperative launch.
+// Resident blocks per SM of a kernel of kSweepThreads threads that needs a
+// cooperative launch; 0 when the device has none.
+template <class Kernel>
+int coop_blocks_per_sm(int device, Kernel kern, size_t smem) {
+    int coop = 0, nb = 0;
+    cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
+    if (coop == 0 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kSweepThreads,
+                                                                   smem) != cudaSuccess) {
+        cudaGetLastError();
+        nb = 0;
+    }
+    return nb;
+}
+
+// Resident k_sweeps blocks per SM (without / with the CTA-role tiles).
 int sweeps_per_sm(int device, bool tiles) {
-    static int cached[64][2];
-    static bool done[64][2];
-    if (device < 0 || device >= 64) {
-        return 0;
-    }
-    if (!done[device][tiles]) {
-        int coop = 0, nb = 0;
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
-        if (coop == 0 ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_sweeps, kSweepThreads,
-                                                          tiles ? smem_tiles(4) : 0) !=
-                cudaSuccess) {
-            cudaGetLastError();
-            nb = 0;
-        }
-        cached[device][tiles] = nb;
-        done[device][tiles] = true;
-    }
-    return cached[device][tiles];
+    static DeviceCache<int> cache[2];
+    return cache[tiles].get(device, [tiles](int dev) {
+        return coop_blocks_per_sm(dev, k_sweeps, tiles ? smem_tiles(4) : 0);
+    });
 }
 
 // Roots, Loewner weights, rows and placement of level a.k: one cooperative
@@ -609,26 +597,10 @@ int launch_sweeps(brdc_handle h, const HostForest &hf, const KArgs &a, cudaStrea
     return 1;
 }
 
-// Resident k_box blocks per SM, once per device; 0 when the device has no
-// cooperative launch.
+// Resident k_box blocks per SM.
 int box_per_sm(int device) {
-    static int cached[64];
-    static bool done[64];
-    if (device < 0 || device >= 64) {
-        return 0;
-    }
-    if (!done[device]) {
-        int coop = 0, nb = 0;
-        cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device);
-        if (coop == 0 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-                             &nb, k_box, kSweepThreads, 0) != cudaSuccess) {
-            cudaGetLastError();
-            nb = 0;
-        }
-        cached[device] = nb;
-        done[device] = true;
-    }
-    return cached[device];
+    static DeviceCache<int> cache;
+    return cache.get(device, [](int dev) { return coop_blocks_per_sm(dev, k_box, 0); });
 }
 
 // The merges of level a.k that k_level leaves: one cooperative k_box.
@@ -662,7 +634,7 @@ int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, boo
     const int mmax = hf.level_mmax[k];
     // a cluster per node: at least one CTA per kLvlRowsPerCta rows, then
     // larger while every node's cluster still runs in the first wave
-    const int *act = level_clusters(h->device);
+    const std::array<int, 5> act = level_clusters(h->device);
     int q = 0;
     while (q < 4 && (1 << q) < h->defl_cluster && act[q + 1] > 0 &&
            (1 << q) * kLvlRowsPerCta < mmax) {

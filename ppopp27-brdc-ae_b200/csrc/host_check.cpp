@@ -1,8 +1,13 @@
 // host_check.cpp -- the product's per-root secular state machine
 // (brdc_secular.cuh) compiled for the host, so the CPU test suite can check
 // its numerics against LAPACK DLAED4 without a GPU.  Not used by the solver.
+#include <atomic>
 #include <cfloat>
+#include <chrono>
+#include <thread>
+#include <vector>
 
+#include "brdc_device_cache.h"
 #include "brdc_leaf.cuh"
 #include "brdc_secular.cuh"
 
@@ -138,4 +143,30 @@ extern "C" int brdc_host_leaf(int s, const double *d, const double *e, double *l
     stats[0] = res;
     stats[1] = orth;
     return res <= kLeafResid && orth <= kLeafOrth;
+}
+
+// `threads` threads ask a device's cache at once; how often the (slow) query
+// ran, or -1 if a thread got another answer than the query's.
+extern "C" int brdc_host_cache_queries(int threads, int device) {
+    brdc::DeviceCache<int> cache;
+    std::atomic<int> queries{0}, wrong{0}, ready{0};
+    std::vector<std::thread> pool;
+    for (int t = 0; t < threads; ++t) {
+        pool.emplace_back([&]() {
+            ++ready;
+            while (ready.load() < threads) {
+            }
+            const int got = cache.get(device, [&](int dev) {
+                std::this_thread::sleep_for(std::chrono::milliseconds(20));
+                ++queries;
+                return 100 + dev;
+            });
+            const bool known = device >= 0 && device < brdc::kMaxDevices;
+            wrong += got != (known ? 100 + device : 0);
+        });
+    }
+    for (std::thread &t : pool) {
+        t.join();
+    }
+    return wrong.load() != 0 ? -1 : queries.load();
 }
