@@ -196,12 +196,12 @@ __global__ void __launch_bounds__(kSweepThreads) k_bw_roots(BArgs a) {
                 if (i == o) {
                     continue;
                 }
-                const double r = brdc_rcp((__ldg(pd + i) - dorg) - tau);
-                const double u = __ldg(zz + i) * r;
+                const double r = brdc_rcp((pd[i] - dorg) - tau);
+                const double u = zz[i] * r;
                 S2x += u * u;
                 S3x += u * u * r;
                 if (!top) {
-                    const double fi = __ldg(pf + i), li = __ldg(pl + i);
+                    const double fi = pf[i], li = pl[i];
                     ax += fi * u;
                     bx += li * u;
                     A2x += fi * u * r;
@@ -297,10 +297,10 @@ __global__ void __launch_bounds__(kSweepThreads) k_bw_poles(BArgs a) {
                     if (j == sk0 || j == sk1) {
                         continue;
                     }
-                    const double r = brdc_rcp((di - __ldg(rdo + j)) - __ldg(rtau + j));
-                    const double in = __ldg(rin + j);
+                    const double r = brdc_rcp((di - rdo[j]) - rtau[j]);
+                    const double in = rin[j];
                     const double u = zi * r * in;
-                    const double kj = __ldg(rk + j);
+                    const double kj = rk[j];
                     gd += u * u * kj;
                     gz -= 2.0 * u * kj * in;
                 }
@@ -312,12 +312,12 @@ __global__ void __launch_bounds__(kSweepThreads) k_bw_poles(BArgs a) {
                     if (j == sk0 || j == sk1) {
                         continue;
                     }
-                    const double r = brdc_rcp((di - __ldg(rdo + j)) - __ldg(rtau + j));
-                    const double in = __ldg(rin + j);
+                    const double r = brdc_rcp((di - rdo[j]) - rtau[j]);
+                    const double in = rin[j];
                     const double u = zi * r * in;
-                    const double kj = __ldg(rk + j);
-                    const double gfj = __ldg(bf + j), glj = __ldg(bl + j);
-                    const double q = gfj * fi + glj * li - u * __ldg(rh + j);
+                    const double kj = rk[j];
+                    const double gfj = bf[j], glj = bl[j];
+                    const double q = gfj * fi + glj * li - u * rh[j];
                     gd += u * (u * kj - q * r);
                     gz += in * (q * r - 2.0 * u * kj);
                     gF += gfj * u;
@@ -452,10 +452,10 @@ __global__ void __launch_bounds__(256) k_bw_defl(BArgs a, long long total_n, int
         if (act) {
 #pragma unroll 4
             for (int j = l; j < Kr; j += tpr) {
-                const double r = brdc_rcp((d - __ldg(w.rdo + pr + j)) - __ldg(w.rtau + pr + j));
-                const double tt = __ldg(w.bfr + pr + j) * f + __ldg(w.blr + pr + j) * e -
-                                  gf * __ldg(w.rfp + pr + j) - gl * __ldg(w.rlp + pr + j);
-                acc += __ldg(w.rinvn + pr + j) * r * (sm ? tt : -tt * r);
+                const double r = brdc_rcp((d - w.rdo[pr + j]) - w.rtau[pr + j]);
+                const double tt = w.bfr[pr + j] * f + w.blr[pr + j] * e -
+                                  gf * w.rfp[pr + j] - gl * w.rlp[pr + j];
+                acc += w.rinvn[pr + j] * r * (sm ? tt : -tt * r);
             }
         }
         acc = group_sum(acc, tpr);

@@ -75,6 +75,9 @@ inline int tree_levels(long long n) {
 // are then already held, so the early CTAs only take what is left), and
 // waits until the previous kernel has finished and its writes are visible.
 // For a kernel launched without the attribute the wait returns at once.
+// A kernel launched with it starts while its inputs are still being written,
+// so it reads them by ordinary loads: the read-only path (__ldg) is for memory
+// that nothing writes while the kernel runs, its wait included.
 __device__ __forceinline__ void pdl_begin() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");

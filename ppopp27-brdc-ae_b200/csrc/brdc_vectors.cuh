@@ -220,9 +220,9 @@ __global__ void __launch_bounds__(256) k_vec_build(VArgs a, long long total_n) {
 #pragma unroll
                 for (int q = 0; q < kVecBatch; ++q) {
                     const int r = b + 32 * q;
-                    v[q] = r < r1 ? __ldg(c + (r - r0)) : 0.0;
+                    v[q] = r < r1 ? c[r - r0] : 0.0;
                     if (a.top && r < r1) {
-                        v[q] *= __ldg(a.sgn + r);
+                        v[q] *= a.sgn[r];
                     }
                 }
 #pragma unroll
