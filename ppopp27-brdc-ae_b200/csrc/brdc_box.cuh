@@ -15,9 +15,10 @@
 // root once and 200 a sweep.  Differences are taken from mid, which
 // is exact to the rounding of the difference, so nothing is lost where a box
 // is narrow.  A box whose far part would be less than half of the poles
-// (clusters straddled by its interval) sums all of them directly.  The last
-// root, whose bracket leaves the poles' range, is summed directly by a whole
-// block.
+// (clusters straddled by its interval) sums all of them directly.  Boxes with
+// many near poles are listed, and their roots get more lanes (box_runs).  The
+// last root, whose bracket leaves the poles' range, is summed directly by a
+// whole block.
 //
 // Bound: FP64 arithmetic.  Measured on B200 against sweeps over all poles
 // (k_sweeps, which still serves levels with the fused kernel off): Toeplitz
@@ -38,11 +39,13 @@ constexpr int kBoxNodes = 6;
 constexpr int kBoxHalves = (kSweepThreads / 32) * kBoxNodes / kBoxP;
 static_assert(kBoxHalves * kBoxP == (kSweepThreads / 32) * kBoxNodes, "points and halves");
 constexpr double kBoxFar = 3.0;  // far: at least this many h from mid
+constexpr int kBoxLong = 6;      // listed: more near poles than this many boxes'
 
 // A box's scratch lies in the node's slices of the next level's arrays,
 // which the placement fills last: 64 doubles of each from the box's first
 // pole on (a box has at least 64 poles).
-//   nd  0 psi, 24 dpsi, 48 mid, 49 1/h, 50 nlo, 51 nhi, 52 h
+//   nd  0 psi, 24 dpsi, 48 mid, 49 1/h, 50 nlo, 51 nhi, 52 h,
+//       53 (of the level's i-th box) the i-th listed box
 //   nf  0 phi, 24 dphi; for the rows 0 sum l u
 //   nl  0 Loewner product; for the rows 0 sum u^2, 24 sum f u
 struct BoxHdr {
@@ -52,7 +55,16 @@ struct BoxHdr {
     // the Loewner product pairs pole j with root j in (d_j, d_{j+1}): the
     // root of the last far pole below may be near
     __device__ int low() const { return nlo > 0 ? nlo - 1 : 0; }
+    __device__ bool listed(int b) const { return nhi - nlo > kBoxLong * b; }
 };
+
+// Where box `item` of the level keeps its scratch.
+__device__ inline long long box_slice(const KArgs &a, int item) {
+    const Ws &w = a.w;
+    const int g = w.items_c[item];
+    return node_geom(a.F, a.k, g).gstart +
+           (long long)(item - w.pref_c[g]) * w.hdr->lvl[a.k].box;
+}
 
 __device__ inline BoxHdr box_header(const Ws &w, long long sb) {
     BoxHdr H;
@@ -112,7 +124,7 @@ __device__ inline int box_count(const double *d, int K, double mid, double v, bo
 template <BoxSum WHAT>
 __device__ void box_far(const KArgs &a, BoxSmem &S) {
     const Ws &w = a.w;
-    const LevelCtl *ctl = &w.hdr->lvl[a.k];
+    LevelCtl *ctl = &w.hdr->lvl[a.k];
     const int boxes = ctl->items_c, b = ctl->box;
     const int warp = threadIdx.x >> 5;
     const int node0 = (warp / kBoxHalves) * kBoxNodes, half = warp % kBoxHalves;
@@ -148,6 +160,9 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
                 w.nd[sb + 50] = (double)H.nlo;
                 w.nd[sb + 51] = (double)H.nhi;
                 w.nd[sb + 52] = H.h;
+                if (H.listed(b)) {
+                    w.nd[box_slice(a, atomicAdd(&ctl->citem, 1)) + 53] = (double)item;
+                }
             }
         } else {
             H = box_header(w, sb);
@@ -266,16 +281,27 @@ __device__ void box_far(const KArgs &a, BoxSmem &S) {
 }
 
 // A warp's share of the near phases: runs of 32 / tpr consecutive poles or
-// roots of one box.  body(G, K, r0, box header, far, lane group, lane).
+// roots of one box.  body(G, g, K, first root, roots, tpr, slice, box header).
+//
+// The listed boxes have runs of their own, with as many lanes per root as the
+// grid has threads for them, up to a warp a root: with the level's lanes, one
+// box whose interval straddles two clusters held up the level, its warps at K
+// terms a sweep for many roots each and the rest of the GPU idle.  Measured on
+// B200 (whole solves, without -> with): poles in two clusters, n = 3000 661 ->
+// 568 us, 40,000 18.5 -> 3.6 ms; in 16 clusters, 9001 1816 -> 1480 us.
 template <class Body>
 __device__ inline void box_runs(const KArgs &a, bool inner_only, Body body) {
     const Ws &w = a.w;
     const LevelCtl *ctl = &w.hdr->lvl[a.k];
-    const int tpr = ctl->tpr_w, items = ctl->items_w, b = ctl->box, Rw = 32 / tpr;
+    const int listed = __ldcg(&ctl->citem), b = ctl->box;
     const int warp = threadIdx.x >> 5;
-    for (int it = (int)blockIdx.x * kWarpsPerBlock + warp; it < items;
+    int tpr = ctl->tpr_w, Rw = 32 / tpr;
+    const int items = ctl->items_w;
+    // the last blocks first: the merges' last roots are with the first ones
+    // (Toeplitz 2049 326 -> 306 us, 4096 437 -> 417)
+    const int back = (int)(gridDim.x - 1 - blockIdx.x);
+    for (int it = back * kWarpsPerBlock + warp; it < items;
          it += (int)gridDim.x * kWarpsPerBlock) {
-        // from the end: the blocks with the merges' last roots come last
         const int item = items - 1 - it;
         const int g = w.items_w[item];
         const NodeGeom G = node_geom(a.F, a.k, g);
@@ -284,6 +310,33 @@ __device__ inline void box_runs(const KArgs &a, bool inner_only, Body body) {
         }
         const int K = w.nK[g], r0 = (item - w.pref_w[g]) * Rw;
         const long long sb = G.gstart + (long long)min(r0 / b, K / b - 1) * b;
+        const BoxHdr H = box_header(w, sb);
+        if (!H.listed(b)) {
+            body(G, g, K, r0, Rw, tpr, sb, H);
+        }
+    }
+    if (listed == 0) {
+        return;
+    }
+    while (tpr < 32 && 2LL * tpr * listed * b <= (long long)gridDim.x * kSweepThreads) {
+        tpr <<= 1;
+    }
+    // a merge's last box has up to 2 b - 1 poles; the first blocks, which had
+    // the fewest runs above, come first, and block 0 last
+    Rw = 32 / tpr;
+    const int per = 2 * b / Rw;
+    const int turn = (int)(blockIdx.x > 0 ? blockIdx.x : gridDim.x) - 1;
+    for (int it = turn * kWarpsPerBlock + warp; it < listed * per;
+         it += (int)gridDim.x * kWarpsPerBlock) {
+        const int item = (int)__ldcg(w.nd + box_slice(a, it / per) + 53);
+        const int g = w.items_c[item];
+        const NodeGeom G = node_geom(a.F, a.k, g);
+        const int K = w.nK[g], q = item - w.pref_c[g];
+        const int r0 = q * b + it % per * Rw;
+        if ((inner_only && G.depth == 0) || r0 >= (q == K / b - 1 ? K : (q + 1) * b)) {
+            continue;
+        }
+        const long long sb = G.gstart + (long long)q * b;
         body(G, g, K, r0, Rw, tpr, sb, box_header(w, sb));
     }
 }

@@ -94,7 +94,8 @@ struct LevelCtl {
     int nbig;        // merges k_level left to k_box (K > kLvlMaxK)
     unsigned bar_count; // grid barrier of k_sweeps and k_box: arrivals, generation
     unsigned bar_gen;
-    int citem;       // next CTA-role item of the secular phase (taken by atomicAdd)
+    int citem;       // k_sweeps: next CTA-role item of the secular phase (taken by
+                     // atomicAdd); k_box: boxes it has listed
     int box;         // poles per box of the merges k_box takes
     double work_w;   // pole-root pairs (sum K^2) of the warp-role merges
     double work_c;   // and of the CTA-role merges
