@@ -255,8 +255,8 @@ typedef struct brdc_timings {
  *                       poles, placement; larger merges continue in the
  *                       sweep kernel); 0 disables it
  * brdc_autotune picks them by timing; defaults: subtree_levels = -1 (a
- * batch of at least 112 rows per SM: 5 with at least 1024 rows per SM and
- * per instance, else 4; otherwise by tree height: 3 up to n = 32768, 5
+ * batch of at least 112 rows per SM: 5 with at least 432 rows per SM and
+ * 1024 per instance, else 4; otherwise by tree height: 3 up to n = 32768, 5
  * above), 16, 303104,
  * fused_level_rows = 2^30 (every level). */
 typedef struct brdc_tuning {

@@ -501,18 +501,20 @@ void mark(brdc_handle h, int slot) {
 
 // Subtree depth of a solve: the handle's setting, or by default the depth
 // measured fastest on B200.  Batches (us a solve at depths 3, 4, 5): 64
-// instances up to 300 rows (7,000 rows) 153, 165, 181; up to 4000 rows
-// (47,000) 412, 332, 355; 1000 up to 500 rows (168,000) 787, 606, 792; so 4
-// once their 256-row subtrees come near half the SMs.  Large batches of long
-// instances, of all families mixed (5.8 million rows, 1400 a matrix) 48,052,
-// 36,601, 35,399: 5.  A single matrix goes by its height: 3 up to 11 levels
-// (n <= 32768), 5 above.
+// instances up to 300 rows (7,000 rows) 153, 165, 181; 4 of 4096 277, 290,
+// 328; up to 4000 rows (47,000) 412, 332, 355; 1000 up to 500 rows (168,000)
+// 787, 606, 792; so 4 once their 256-row subtrees come near half the SMs.
+// With long instances 5 from about 64,000 rows on: 8 of 4096 308, 309, 339,
+// 16 of 4000 438, 358, 345, 2 of 40,000 910, 760, 753 (clustered 908, 698,
+// 649), all families mixed (5.8 million rows, 1400 a matrix) 48,052, 36,601,
+// 35,399; with short ones not: 500 of 200 447, 305, 454.  A single matrix
+// goes by its height: 3 up to 11 levels (n <= 32768), 5 above.
 int effective_sub_levels(brdc_handle h, const HostForest &hf) {
     if (h->sub_levels >= 0) {
         return h->sub_levels;
     }
     if (hf.B > 1 && hf.total_n >= 112LL * h->sm_count) {
-        return hf.total_n >= 1024LL * std::max(h->sm_count, hf.B) ? 5 : 4;
+        return hf.total_n >= std::max(432LL * h->sm_count, 1024LL * hf.B) ? 5 : 4;
     }
     // measured on B200 (uniform and normal, ms per solve): depth 3 is the
     // fastest up to n = 32,768 (11 levels; 32,768: 0.583 against 0.609 at
@@ -646,10 +648,12 @@ int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, boo
     const int C = 1 << q;
     KArgs a = a0;
     // k_box takes merges with more than kBoxMinK poles on the levels that
-    // launch it: those of a batch, where one more launch is nothing, and those
-    // that may hold merges k_level cannot take.  (Launched for nothing it
-    // costs a level 4 us.)
-    const bool big = mmax > (hf.B > 1 ? kBoxMinK : kLvlMaxK);
+    // launch it: those that may hold merges k_level cannot take, and those of
+    // a batch with too many merges for k_level's largest clusters.  (Launched
+    // for nothing it costs a level 4 us.  Batches whose matrices deflate
+    // little, us without and with it: 4 of 700 rows 209, 224, 4 of 1000 276,
+    // 276, 8 of 1000 336, 300, 16 of 1000 438, 340.)
+    const bool big = mmax > kLvlMaxK || (hf.B > 1 && a.nodes >= kBoxMinNodes && mmax > kBoxMinK);
     a.big_k = big ? kBoxMinK : kLvlMaxK;
     a.keep = ckpt ? 1 : 0;
     a.plan_inline = big && a.nodes <= kLvlThreads ? 1 : 0;

@@ -616,6 +616,7 @@ __host__ __device__ inline int box_poles(int kmax) {
 // the terms, and every SM shares them (Toeplitz 16,384 1.37 ms at 1024, 1.30
 // at 512 and at 256; a batch of 512 up to 2048 rows 2.10, 1.66, 1.63 ms).
 constexpr int kBoxMinK = 512;
+constexpr int kBoxMinNodes = 8; // merges of a batch's level of up to kLvlMaxK rows it runs for
 // Lanes per root there at most: a lane should have two dozen of the 3 b near
 // poles (Toeplitz 16,384, two merges of 8192 poles: 860 us at 16 lanes, 798
 // at 8, 750 at 4; one of 4096 poles is faster at 8).
