@@ -1183,7 +1183,7 @@ def work_model(diag, fused):
         sweeps = lv["secular_iter_sum"] / kk + 1.0
         far, near = 0.0, float(lv["dd_after_sq_sum"])
         kmax = lv["dd_after_max"]
-        if kmax > 512 and lv["size_sum"] > 1024 * lv["merge_count"]:
+        if kmax > (768 if lv["merge_count"] < 64 else 512) and lv["size_sum"] > 1024 * lv["merge_count"]:
             # k_box: 24 points per box of b poles for the far sums, once, and
             # the near poles, about 3 b
             b = 64 if kmax <= 8192 else 128 if kmax <= 16384 else 256

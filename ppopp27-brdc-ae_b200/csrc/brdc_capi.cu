@@ -647,14 +647,14 @@ int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, boo
     }
     const int C = 1 << q;
     KArgs a = a0;
-    // k_box takes merges with more than kBoxMinK poles on the levels that
-    // launch it: those that may hold merges k_level cannot take, and those of
-    // a batch with too many merges for k_level's largest clusters.  (Launched
-    // for nothing it costs a level 4 us.  Batches whose matrices deflate
-    // little, us without and with it: 4 of 700 rows 209, 224, 4 of 1000 276,
-    // 276, 8 of 1000 336, 300, 16 of 1000 438, 340.)
-    const bool big = mmax > kLvlMaxK || (hf.B > 1 && a.nodes >= kBoxMinNodes && mmax > kBoxMinK);
-    a.big_k = big ? kBoxMinK : kLvlMaxK;
+    // k_box runs on the levels that may hold merges k_level cannot take, and on
+    // those of a batch with too many merges for k_level's largest clusters.
+    // (Launched for nothing it costs a level 4 us.  Batches whose matrices
+    // deflate little, us without and with it: 4 of 1000 rows 276, 276, 8 of
+    // 1000 336, 300, 16 of 1000 438, 340.)
+    const int box_k = a.nodes < kBoxManyNodes ? kBoxMinKFew : kBoxMinK;
+    const bool big = mmax > kLvlMaxK || (hf.B > 1 && a.nodes >= kBoxMinNodes && mmax > box_k);
+    a.big_k = big ? box_k : kLvlMaxK;
     a.keep = ckpt ? 1 : 0;
     a.plan_inline = big && a.nodes <= kLvlThreads ? 1 : 0;
     cudaLaunchAttribute at[2];

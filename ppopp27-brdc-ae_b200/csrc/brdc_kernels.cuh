@@ -612,10 +612,18 @@ constexpr int kWarpsPerBlock = kSweepThreads / 32;
 __host__ __device__ inline int box_poles(int kmax) {
     return kmax <= 8192 ? 64 : kmax <= 16384 ? 128 : 256;
 }
-// Merges of more poles than this are k_box's where it runs: it takes half
-// the terms, and every SM shares them (Toeplitz 16,384 1.37 ms at 1024, 1.30
-// at 512 and at 256; a batch of 512 up to 2048 rows 2.10, 1.66, 1.63 ms).
+// Merges of more poles than kBoxMinK are k_box's where it runs: it takes half
+// the terms, and every SM shares them (100 Toeplitz matrices of 1060 rows, 530
+// poles, 1459 us in k_level, 1277 in k_box, of 1400 rows 1802, 1427; a batch of
+// 512 up to 2048 rows 2.10 ms at 1024, 1.66 at 512, 1.63 at 256).  A level of
+// fewer than kBoxManyNodes merges leaves most SMs to either kernel, and k_box
+// comes after k_level and waits at its grid barriers: up to kBoxMinKFew poles
+// stay in k_level (4 Toeplitz of 1060 rows 305 us in k_box, 265 in k_level, of
+// 1400 330, 306, 32 of 1400 679, 640, but 8 of 1520 365, 386; of 1600 rows, 800
+// poles: 4 339, 342, 8 376, 429, 32 720, 772; glued W21 of 3000 633, 551).
 constexpr int kBoxMinK = 512;
+constexpr int kBoxMinKFew = 768;
+constexpr int kBoxManyNodes = 64;
 constexpr int kBoxMinNodes = 8; // merges of a batch's level of up to kLvlMaxK rows it runs for
 // Lanes per root there at most: a lane should have two dozen of the 3 b near
 // poles (Toeplitz 16,384, two merges of 8192 poles: 860 us at 16 lanes, 798
