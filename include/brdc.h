@@ -171,7 +171,8 @@ typedef struct brdc_level_diagnostics {
     int secular_iter_sum;    /* secular iterations summed over roots */
     int secular_iter_max;
     int secular_iter_failed; /* roots that hit the iteration cap */
-    int threads_per_root;    /* lanes that shared one root's sums */
+    int threads_per_root;    /* lanes that shared one root's sums (on a
+                                checkpointing workspace: the adjoint's) */
     long long dd_after_sq_sum; /* sum of K^2: pole-root pairs of the level */
 } brdc_level_diagnostics;
 
@@ -248,12 +249,17 @@ typedef struct brdc_timings {
  *                       merge (1, 2, 4, 8 or 16; 1 = one CTA per merge; the
  *                       per-level deflation kernel uses at most 8)
  *   sweep_lanes_target  threads the per-level root sweeps aim to keep busy
- *                       (lanes per root = smallest power of two reaching it)
+ *                       (lanes per root = smallest power of two reaching it);
+ *                       the interpolating kernel and the adjoint take a
+ *                       quarter of them
  *   fused_level_rows    levels above the subtree whose largest merge has at
  *                       most this many rows run as one fused kernel per level
- *                       (merge, deflation, roots of merges with <= 1024
- *                       poles, placement; larger merges continue in the
- *                       sweep kernel); 0 disables it
+ *                       (merge, deflation, roots, placement); 0 disables it.
+ *                       A second kernel with interpolated sums finishes the
+ *                       merges that keep many poles: more than 512, or 768 on
+ *                       levels of fewer than 64 merges, on the levels whose
+ *                       largest merge has more than 1024 rows (in a batch,
+ *                       also on smaller ones of 8 or more merges)
  * brdc_autotune picks them by timing; defaults: subtree_levels = -1 (a
  * batch of at least 112 rows per SM: 5 with at least 432 rows per SM and
  * 1024 per instance, else 4; otherwise by tree height: 3 up to n = 32768, 5

@@ -8,8 +8,9 @@
 // a box's interval [mid - h, mid + h] the part of F from the poles at least
 // h * 2 away from the interval is analytic well beyond it (a Bernstein
 // ellipse of parameter 3 + sqrt(8) = 5.83), so its interpolant at p = 24
-// Chebyshev points is exact to 5.83^-24 = 4e-19 of it, below rounding.  A
-// box's interpolants cost p K terms once, and each of its b poles or roots
+// Chebyshev points is off by at most 2.5e-18 of it (one pole at the edge of
+// the far part, evaluated in extended precision; the squared sums, whose poles
+// are double, 3.1e-17), below rounding.  A box's interpolants cost p K terms once, and each of its b poles or roots
 // then takes the near poles (3 b where they lie evenly) and one polynomial
 // per sum and sweep instead of K terms: at K = 4096, b = 64, 1536 terms a
 // root once and 200 a sweep.  Differences are taken from mid, which

@@ -91,7 +91,7 @@ struct LevelCtl {
     int items_w;     // warp work items of the level
     int items_c;     // CTA work items of the level
     int total_k;
-    int nbig;        // merges k_level left to k_box (K > kLvlMaxK)
+    int nbig;        // merges k_level left to k_box (K > KArgs::big_k)
     unsigned bar_count; // grid barrier of k_sweeps and k_box: arrivals, generation
     unsigned bar_gen;
     int citem;       // k_sweeps: next CTA-role item of the secular phase (taken by
@@ -129,9 +129,10 @@ enum DeviceError : int {
 
 // A solve whose status word is set (non-finite input, a wait that ran out)
 // does no further work: every kernel after the one that set it returns at
-// once.  Only k_norm, k_sweeps and k_box set the word, and every later kernel
-// waits for them to finish before it reads it, so all CTAs of a kernel read
-// the same value (no cluster or grid barrier can lose a member to it).
+// once.  Only k_norm, k_sweeps and k_box set the word (k_level too, should a
+// bulk copy never land), and every later kernel waits for them to finish
+// before it reads it, so all CTAs of a kernel read the same value (no cluster
+// or grid barrier can lose a member to it).
 #if defined(__CUDACC__)
 __device__ __forceinline__ bool halted(const WsHeader *h) {
     return *(const volatile int *)&h->status != 0;

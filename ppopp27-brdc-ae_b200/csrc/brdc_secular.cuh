@@ -20,8 +20,9 @@
 //     representation of cpu/src/dlaed4_br.f:15-26,95-103);
 //   * the sweep excludes the two bracketing poles p, p+1; the root adds
 //     their terms itself so they are never cancelled against the rest.
-// The error bound is LAPACK's running-sum bound for the summation order the
-// sweep actually uses.
+// The error bound is LAPACK's running-sum bound for the summation order of the
+// sweep (k_sweeps and k_box's near sums), or the bound that sec_bound forms
+// from the size of the sums (sweeps in shared memory, k_box's last roots).
 #pragma once
 
 #include <cmath>

@@ -126,7 +126,8 @@ constexpr int kVecBatch = 8; // rows a lane of k_vec_build copies at once
 // disjoint rows, so lanes take different chains); the products turn these
 // into the node's root eigenvectors.  A deflated slot is a child
 // eigenvector (small-z) or a short rotation combination of some (rotated
-// out), written straight to its place in the node's block.  M must be zero.
+// out), written straight to its place in the node's block.  M need not be
+// cleared: every row of a root column that k_vec_gemm reads is written here.
 __global__ void __launch_bounds__(256) k_vec_build(VArgs a, long long total_n) {
     pdl_begin();
     if (halted(a.w.hdr)) {
