@@ -1183,7 +1183,8 @@ def work_model(diag, fused):
         sweeps = lv["secular_iter_sum"] / kk + 1.0
         far, near = 0.0, float(lv["dd_after_sq_sum"])
         kmax = lv["dd_after_max"]
-        if kmax > (768 if lv["merge_count"] < 64 else 512) and lv["size_sum"] > 1024 * lv["merge_count"]:
+        rows = -(-lv["size_sum"] // max(lv["merge_count"], 1))
+        if rows > 1024 and kmax > min(1024, max(512, rows // 20 * 9)):
             # k_box: 24 points per box of b poles for the far sums, once, and
             # the near poles, about 3 b
             b = 64 if kmax <= 8192 else 128 if kmax <= 16384 else 256

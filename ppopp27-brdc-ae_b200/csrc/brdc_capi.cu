@@ -648,13 +648,11 @@ int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, boo
     const int C = 1 << q;
     KArgs a = a0;
     // k_box runs on the levels that may hold merges k_level cannot take, and on
-    // those of a batch with too many merges for k_level's largest clusters.
-    // (Launched for nothing it costs a level 4 us.  Batches whose matrices
-    // deflate little, us without and with it: 4 of 1000 rows 276, 276, 8 of
-    // 1000 336, 300, 16 of 1000 438, 340.)
-    const int box_k = a.nodes < kBoxManyNodes ? kBoxMinKFew : kBoxMinK;
-    const bool big = mmax > kLvlMaxK || (hf.B > 1 && a.nodes >= kBoxMinNodes && mmax > box_k);
-    a.big_k = big ? box_k : kLvlMaxK;
+    // those of a batch with too many merges for k_level's largest clusters
+    // (launched for nothing it costs a level 4 us)
+    const int rows = a.nodes < kBoxManyNodes ? kBoxFewRows : kBoxMinK;
+    const bool big = mmax > kLvlMaxK || (hf.B > 1 && a.nodes >= kBoxMinNodes && mmax > rows);
+    a.big_k = big ? box_min_poles(mmax, kLvlMaxK) : kLvlMaxK;
     a.keep = ckpt ? 1 : 0;
     a.plan_inline = big && a.nodes <= kLvlThreads ? 1 : 0;
     cudaLaunchAttribute at[2];

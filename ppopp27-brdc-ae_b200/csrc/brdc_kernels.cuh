@@ -612,19 +612,29 @@ constexpr int kWarpsPerBlock = kSweepThreads / 32;
 __host__ __device__ inline int box_poles(int kmax) {
     return kmax <= 8192 ? 64 : kmax <= 16384 ? 128 : 256;
 }
-// Merges of more poles than kBoxMinK are k_box's where it runs: it takes half
-// the terms, and every SM shares them (100 Toeplitz matrices of 1060 rows, 530
-// poles, 1459 us in k_level, 1277 in k_box, of 1400 rows 1802, 1427; a batch of
-// 512 up to 2048 rows 2.10 ms at 1024, 1.66 at 512, 1.63 at 256).  A level of
-// fewer than kBoxManyNodes merges leaves most SMs to either kernel, and k_box
-// comes after k_level and waits at its grid barriers: up to kBoxMinKFew poles
-// stay in k_level (4 Toeplitz of 1060 rows 305 us in k_box, 265 in k_level, of
-// 1400 330, 306, 32 of 1400 679, 640, but 8 of 1520 365, 386; of 1600 rows, 800
-// poles: 4 339, 342, 8 376, 429, 32 720, 772; glued W21 of 3000 633, 551).
+// Which merges k_box takes, where a level runs it (launch_level_fused): those
+// of more than kBoxMinK poles that keep at least 9/20 of their level's rows.
+// It takes half of k_level's terms, and every SM shares them: 32 merges of
+// 1250 rows, Toeplitz, 284 us with up to 1024 poles in k_level, 191 with up
+// to 512; Toeplitz 44,719 2955 and 2873 us with up to 768 and 629 (100 matrices
+// of 1060 rows 1459 us at 1024, 1277 at 512).  But it runs after k_level, so a
+// level all of whose merges deflate more than half stays there: 2 merges of
+// 1500 rows of glued W21, 569 poles, 124 us in k_level, 208 in k_box; 32 of
+// them 178, 333; so where the merges keep less, up to kLvlMaxK stay.
 constexpr int kBoxMinK = 512;
-constexpr int kBoxMinKFew = 768;
+__host__ __device__ inline int box_min_poles(int mmax, int most) {
+    const int k = mmax / 20 * 9;
+    return k < kBoxMinK ? kBoxMinK : k < most ? k : most;
+}
+// Levels of a batch of up to kLvlMaxK rows run it from kBoxMinNodes merges of
+// more than kBoxFewRows rows on, of more than kBoxMinK from kBoxManyNodes on.
+// Us of the level in k_level and in k_box: 4 merges of 1000 rows that deflate
+// little 76, 75, 8 115, 81, 32 217, 133; of 750 rows 8 84, 77, 32 143, 126,
+// 128 444, 294, but inner merges of 750 rows 8 110, 114, 32 184, 196, and
+// Toeplitz ones 90, 133 and 137, 167.
+constexpr int kBoxMinNodes = 8;
 constexpr int kBoxManyNodes = 64;
-constexpr int kBoxMinNodes = 8; // merges of a batch's level of up to kLvlMaxK rows it runs for
+constexpr int kBoxFewRows = 768;
 // Lanes per root there at most: a lane should have two dozen of the 3 b near
 // poles (Toeplitz 16,384, two merges of 8192 poles: 860 us at 16 lanes, 798
 // at 8, 750 at 4; one of 4096 poles is faster at 8).
