@@ -459,18 +459,20 @@ __device__ double level_poles(LvlSmem &S, cooperative_groups::cluster_group &cl,
     v.gs = writer ? w.gs + gs : S.stage + kLvlMaxK;
     v.gr = writer ? w.gr + gs : S.stage + 2 * kLvlMaxK;
     const bool rot = __syncthreads_or(defl_close_walk<T>(v, 0, Kz, tol, 0, Kz));
-    if (keep && loaded && rot) {
-        cl.sync();
-    }
-    if (writer && keep && (rot || !loaded)) {
-        // what the adjoint and the vectors read of the list (d and z are not
-        // among it)
-        for (int i = x; i < Kz; i += T) {
-            w.af[gs + i] = S.pf[i];
-            w.al[gs + i] = S.pl[i];
-            w.amap[gs + i] = S.amap[i];
-            w.gmark[gs + i] = S.gmark[i];
-            w.gbase[gs + i] = S.gbase[i];
+    if (keep) {
+        if (loaded && rot) {
+            cl.sync();
+        }
+        if (writer && (rot || !loaded)) {
+            // what the adjoint and the vectors read of the list (d and z are
+            // not among it)
+            for (int i = x; i < Kz; i += T) {
+                w.af[gs + i] = S.pf[i];
+                w.al[gs + i] = S.pl[i];
+                w.amap[gs + i] = S.amap[i];
+                w.gmark[gs + i] = S.gmark[i];
+                w.gbase[gs + i] = S.gbase[i];
+            }
         }
     }
     int K = Kz;
