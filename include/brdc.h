@@ -256,8 +256,9 @@ typedef struct brdc_timings {
  *                       most this many rows run as one fused kernel per level
  *                       (merge, deflation, roots, placement); 0 disables it.
  *                       A second kernel with interpolated sums finishes the
- *                       merges that keep many poles (more than 512 and 9/20
- *                       of their rows, or more than 1024) on the levels whose
+ *                       merges that keep many poles (more than 512, and on a
+ *                       level of fewer than 64 merges 9/20 of their rows, or
+ *                       more than 1024) on the levels whose
  *                       largest merge has more than 1024 rows (in a batch, also
  *                       8 merges of more than 768 rows or 64 of more than 512)
  * brdc_autotune picks them by timing; defaults: subtree_levels = -1 (a

@@ -650,9 +650,10 @@ int launch_level_fused(brdc_handle h, const HostForest &hf, const KArgs &a0, boo
     // k_box runs on the levels that may hold merges k_level cannot take, and on
     // those of a batch with too many merges for k_level's largest clusters
     // (launched for nothing it costs a level 4 us)
-    const int rows = a.nodes < kBoxManyNodes ? kBoxFewRows : kBoxMinK;
-    const bool big = mmax > kLvlMaxK || (hf.B > 1 && a.nodes >= kBoxMinNodes && mmax > rows);
-    a.big_k = big ? box_min_poles(mmax, kLvlMaxK) : kLvlMaxK;
+    const bool many = a.nodes >= kBoxManyNodes;
+    const bool big = mmax > kLvlMaxK || (hf.B > 1 && a.nodes >= kBoxMinNodes &&
+                                         mmax > (many ? kBoxMinK : kBoxFewRows));
+    a.big_k = !big ? kLvlMaxK : many ? kBoxMinK : box_min_poles(mmax, kLvlMaxK);
     a.keep = ckpt ? 1 : 0;
     a.plan_inline = big && a.nodes <= kLvlThreads ? 1 : 0;
     cudaLaunchAttribute at[2];

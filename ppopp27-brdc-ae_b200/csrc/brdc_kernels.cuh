@@ -620,7 +620,9 @@ __host__ __device__ inline int box_poles(int kmax) {
 // of 1060 rows 1459 us at 1024, 1277 at 512).  But it runs after k_level, so a
 // level all of whose merges deflate more than half stays there: 2 merges of
 // 1500 rows of glued W21, 569 poles, 124 us in k_level, 208 in k_box; 32 of
-// them 178, 333; so where the merges keep less, up to kLvlMaxK stay.
+// them 178, 333; so where the merges keep less, up to kLvlMaxK stay, unless
+// the level has kBoxManyNodes (4096 matrices of all families 35.9 ms with the
+// share asked for there too, 35.5 without).
 constexpr int kBoxMinK = 512;
 __host__ __device__ inline int box_min_poles(int mmax, int most) {
     const int k = mmax / 20 * 9;
